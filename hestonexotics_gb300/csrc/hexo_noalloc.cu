@@ -92,8 +92,8 @@ hexo_status na_setup(int dev, bool f32, unsigned char **scratch, uint32_t *grid_
         int sms = 0;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
             return HEXO_ERR_CUDA;
-        const size_t smem = paths_smem_bytes(kNaBlock, 1);
         for (int k = 0; k < 2; ++k) {
+            const size_t smem = paths_smem_bytes(k == 1, kNaBlock, 1);
             const void *fn = paths_kernel_ptr(k == 1, 1, 1);
             int nb = 0;
             if (paths_smem_limit(fn, dev) != cudaSuccess ||
@@ -121,11 +121,11 @@ SegDesc na_segment(const hexo_params &p, double dt) {
     s.K1 = 0.5 * dt * (p.kappa * p.rho / p.sigma - 0.5) - p.rho / p.sigma;
     s.K2 = 0.5 * dt * (p.kappa * p.rho / p.sigma - 0.5) + p.rho / p.sigma;
     s.K3 = 0.5 * dt * (1.0 - p.rho * p.rho);
-    s.K4 = 0.5 * dt * (1.0 - p.rho * p.rho);
+    s.m0 = p.theta * (1.0 - s.disc);
     s.hdt = dt * 0.5;
     s.f_disc = (float)s.disc; s.f_cA = (float)s.cA; s.f_cB = (float)s.cB;
     s.f_K0 = (float)s.K0; s.f_K1 = (float)s.K1; s.f_K2 = (float)s.K2;
-    s.f_K3 = (float)s.K3; s.f_K4 = (float)s.K4; s.f_hdt = (float)s.hdt;
+    s.f_K3 = (float)s.K3; s.f_K4 = (float)s.K3; s.f_hdt = (float)s.hdt;
     s.f_c = (float)(0.5 * dt * (p.kappa * p.rho / p.sigma - 0.5));
     ds_split(s.disc, s.ds_disc);
     ds_split(p.theta * (1.0 - s.disc), s.ds_m0);
@@ -328,7 +328,7 @@ extern "C" hexo_status hexo_price_noalloc(const hexo_params *pp, double S0, cons
     a.n_opts = n_opts;
     const LaunchShape sh{kNaBlock, 1, 1};
     const uint32_t grid = std::max<uint32_t>(1, std::min(slots, n_tiles));
-    if (e == cudaSuccess && n_tiles > 0) e = launch_paths(f32, sh, grid, paths_smem_bytes(kNaBlock, 1), s, a);
+    if (e == cudaSuccess && n_tiles > 0) e = launch_paths(f32, sh, grid, paths_smem_bytes(f32, kNaBlock, 1), s, a);
     double *d_price = reinterpret_cast<double *>(base + kOffPrice);
     double *d_se = reinterpret_cast<double *>(base + kOffSe);
     if (e == cudaSuccess) {

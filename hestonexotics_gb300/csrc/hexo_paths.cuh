@@ -20,6 +20,7 @@
 #include "hexo_types.h"
 #include "hexo_device.cuh"
 #include "hexo_ds.cuh"
+#include "hexo_f64.cuh"
 
 namespace hexo {
 
@@ -46,45 +47,32 @@ struct PathVars {
 // bits for the same path.
 
 // One QE step of one path (HSimulation.tpp:52-86), FP64; returns whether it
-// took the quadratic branch.
-__device__ __forceinline__ bool qe_step(PathVars<false> &pv, const SegDesc &sg, double theta, dev::Shishua &g,
-                                        dev::RngLane &c, const dev::Ring &r, const dev::WarpScratch &ws) {
+// took the quadratic branch.  The FP64 pipe bounds it: about 100 instructions
+// a step as the reference writes it, 20 (quadratic) or 23 (exponential) with
+// the roots, quotients, log and exp of hexo_f64.cuh.
+__device__ __forceinline__ bool qe_step(PathVars<false> &pv, const SegDesc &sg, const double &theta, dev::Shishua &g,
+                                        dev::RngLane &c, const dev::Ring &r, const dev::WarpScratch &ws,
+                                        const f64::ExpTab *etab) {
     dev::DrawPlan dp = dev::draw_prefetch(c, r);
     const double v = pv.v;
-    const double m = __fma_rn(__dsub_rn(v, theta), sg.disc, theta);         // tpp:59
-    const double sp2 = fabs(__fma_rn(v, sg.cA, sg.cB));                      // tpp:60
-    const double mm = __dmul_rn(m, m);
-    const bool quad = sp2 < __dmul_rn(1.5, mm);                              // Psi < PSI_C, tpp:61,63
+    const double m = __fma_rn(v, sg.disc, sg.m0);                            // tpp:59
+    const double s2 = fabs(__fma_rn(v, sg.cA, sg.cB));                       // tpp:60
+    const bool near = f64::in_range(m, s2);
+    const bool quad = near ? f64::quadratic(m, s2) : s2 < __dmul_rn(1.5, __dmul_rn(m, m));
     if (dev::draw_prepare<false>(g, c, r, ws, quad)) dp = dev::draw_prefetch(c, r);
-    float z1f = 0.0f, z2f;                                                   // draw order, tpp:67,72,80
+    float z1 = 0.0f, z2;                                                     // draw order, tpp:67,72,80
     uint64_t uw = 0;
-    dev::draw_commit(g, c, r, dp, quad, z1f, uw, z2f);
-    const double z1 = (double)z1f;
-    const double z2 = (double)z2f;
+    dev::draw_commit(g, c, r, dp, quad, z1, uw, z2);
     double vn;
-    if (quad) {                                                              // tpp:64-68
-        const double inv = __ddiv_rn(__dmul_rn(2.0, mm), sp2);               // 2/Psi
-        const double im1 = __dsub_rn(inv, 1.0);
-        const double bp2 = __dadd_rn(im1, __dsqrt_rn(__dmul_rn(inv, im1)));
-        const double b = __dsqrt_rn(bp2);
-        const double a = __ddiv_rn(m, __dadd_rn(1.0, bp2));
-        const double zb = __dadd_rn(b, z1);
-        vn = __dmul_rn(__dmul_rn(a, zb), zb);
-    } else {                                                                 // tpp:70-73
-        const double Psi = __ddiv_rn(sp2, mm);
-        const double p = __ddiv_rn(__dsub_rn(Psi, 1.0), __dadd_rn(Psi, 1.0));
-        const double beta = __ddiv_rn(2.0, __dmul_rn(m, __dadd_rn(Psi, 1.0)));
-        const double U = dev::uniform_f64(uw);
-        vn = p < U ? __ddiv_rn(log(__ddiv_rn(__dsub_rn(1.0, p), __dsub_rn(1.0, U))), beta) : 0.0;
-    }
+    if (!near) vn = f64::variance_wide(v, theta, sg.disc, s2, quad, z1, uw);
+    else if (quad) vn = f64::variance_quadratic(m, s2, z1);                  // tpp:64-68
+    else vn = f64::variance_exponential(m, s2, uw);                          // tpp:70-73
     pv.v = vn;
-    double t = __dadd_rn(pv.lx, sg.K0);                                     // tpp:80
-    t = __fma_rn(sg.K1, v, t);
-    t = __fma_rn(sg.K2, vn, t);
-    const double sd = __dsqrt_rn(__fma_rn(sg.K3, v, __dmul_rn(sg.K4, vn)));
-    pv.lx = __fma_rn(sd, z2, t);
+    const double sd = f64::root(__dmul_rn(sg.K3, __dadd_rn(v, vn)));
+    const double t = __fma_rn(sg.K2, vn, __fma_rn(sg.K1, v, __dadd_rn(pv.lx, sg.K0)));   // tpp:80
+    pv.lx = __fma_rn(sd, f64::to_double(z2), t);
     pv.Xp = pv.X;
-    pv.X = exp(pv.lx);                                                       // tpp:82
+    pv.X = f64::exp_tab(pv.lx, etab);                                        // tpp:82
     return quad;
 }
 
@@ -217,9 +205,12 @@ __device__ __forceinline__ void fold_option(const KernelArgs &a, const SetDesc &
                     ok &= dev::limbs_add_signed_f64(d, E, l);
                 } else {
                     const double f = kind == 0u ? asian[p] : (kCV && kind == 2u) ? geo[p] : euro[p];
-                    const double pay = fmax(0.0, __dsub_rn(f, K));
-                    any |= pay != 0.0;
-                    ok &= dev::limbs_add_f64(pay, E, l);
+                    const double pay = __dsub_rn(f, K);
+                    const int64_t bits = __double_as_longlong(pay);
+                    if (bits > 0 && bits <= 0x7ff0000000000000ll) {   // positive; as max(0, pay), a NaN counts as 0
+                        any = true;
+                        ok &= dev::limbs_add_f64(pay, E, l);
+                    }
                 }
             }
         }
@@ -249,9 +240,12 @@ __global__ void __launch_bounds__(512) paths_kernel(const KernelArgs a) {
     uint16_t *tq_i_all = reinterpret_cast<uint16_t *>(nrm_all + (size_t)PPT * 2 * kRngWords * bd);
     uint32_t *win = reinterpret_cast<uint32_t *>(
         smem_raw + ((size_t)PPT * 2 * kRngWords * bd * 12 + (size_t)(bd >> 5) * kWarpScratchBytes + 15) / 16 * 16);
-    // double-single log table of the FP32 form's exponential branch, after the windows
+    // after the windows: the double-single log table of the FP32 form's exponential branch, or the
+    // FP64 form's exponential table; visible after the first tile's barrier
     ds::LogTab *ltab = reinterpret_cast<ds::LogTab *>(win + (size_t)(bd >> 5) * kWindow * kLimbs);
-    if constexpr (kF32) ds::log_table_init(ltab, tid, bd);   // visible after the first tile's barrier
+    f64::ExpTab *etab = reinterpret_cast<f64::ExpTab *>(ltab);
+    if constexpr (kF32) ds::log_table_init(ltab, tid, bd);
+    else f64::exp_table_init(etab, tid, bd);
 
     dev::Ring ring[PPT];
     dev::WarpScratch ws[PPT];
@@ -308,7 +302,6 @@ __global__ void __launch_bounds__(512) paths_kernel(const KernelArgs a) {
         if (!HEXO_CHECK((uint64_t)S.seg_begin + td.seg_count <= a.n_segs && td.seg_count <= S.seg_count, a.error,
                         a.check, kCheckSegs, td.set))
             continue;
-        const double theta = S.theta;
         const float S0f = S.f_S0, rf = S.f_r;
         uint32_t win_base = 0;   // first set option of the staging window
 
@@ -337,6 +330,12 @@ __global__ void __launch_bounds__(512) paths_kernel(const KernelArgs a) {
         for (uint32_t si = 0; si < td.seg_count; ++si) {
             const SegDesc sg = a.segs[S.seg_begin + si];
             const R hdt = kF32 ? (R)sg.f_hdt : (R)sg.hdt;
+            // the FP64 form's trapezoid, one instruction a step: hdt at the
+            // segment's ends, dt at the spots between
+            if constexpr (!kF32)
+                if (sg.n_steps > 1)
+#pragma unroll
+                    for (int p = 0; p < PPT; ++p) pv[p].acc = __fma_rn(hdt, pv[p].X, pv[p].acc);
             // every step, then the trapezoid with this width except after the
             // last (pricing) step; one copy of the step code
 #pragma unroll UNROLL
@@ -344,14 +343,15 @@ __global__ void __launch_bounds__(512) paths_kernel(const KernelArgs a) {
 #pragma unroll
                 for (int p = 0; p < PPT; ++p) {
                     if constexpr (kF32) qe_step(pv[p], sg, g[p], c[p], ring[p], ws[p], S0f, rf, ltab);
-                    else qe_step(pv[p], sg, theta, g[p], c[p], ring[p], ws[p]);
+                    else qe_step(pv[p], sg, S.theta, g[p], c[p], ring[p], ws[p], etab);
                     if constexpr (kCV) {
                         yp[p] = yc[p];   // FP32: the exponent of X / S0 that qe_step used
                         if constexpr (kF32) yc[p] = __fmaf_rn(rf, pv[p].v, pv[p].lx);
                         else yc[p] = __dsub_rn(pv[p].lx, S.logS0);
                     }
                     if (st < sg.n_steps) {
-                        pv[p].acc = fma_r(hdt, add_r(pv[p].X, pv[p].Xp), pv[p].acc);
+                        if constexpr (kF32) pv[p].acc = __fmaf_rn(hdt, __fadd_rn(pv[p].X, pv[p].Xp), pv[p].acc);
+                        else pv[p].acc = __fma_rn(st + 1 < sg.n_steps ? sg.dt : hdt, pv[p].X, pv[p].acc);
                         if constexpr (kCV) accg[p] = fma_r(hdt, add_r(yc[p], yp[p]), accg[p]);
                     }
                 }
