@@ -70,7 +70,7 @@ hexo_status shape_check(hexo_ctx *ctx, bool f32, const LaunchShape &sh, size_t &
     const void *fn = paths_kernel_ptr(f32, sh.ppt, sh.unroll, sh.cv);
     if (fn == nullptr || sh.block == 0 || sh.block % 32 != 0 || sh.block > 512)
         return ctx_fail(ctx, HEXO_ERR_INVALID, "unsupported launch shape (block multiple of 32 up to 512, ppt/unroll in {1,2,4})");
-    smem = paths_smem_bytes(f32, sh.block, sh.ppt);
+    smem = paths_smem_bytes(sh.block, sh.ppt);
     size_t smem_static = 0;
     cudaFuncAttributes fa;
     if (cudaFuncGetAttributes(&fa, fn) == cudaSuccess) smem_static = fa.sharedSizeBytes;
@@ -685,7 +685,7 @@ hexo_status hexo_plan_schedule(const hexo_params *p, double S0, const hexo_optio
     *n_mats = (uint32_t)sp.mats.size();
     for (uint32_t j = 0; j < *n_mats && j < cap; ++j) {
         if (steps_to_mat) steps_to_mat[j] = sp.steps_to_mat[j];
-        if (tmtp) tmtp[j] = sp.mats[j].tmtp;
+        if (tmtp) tmtp[j] = sp.mat_tmtp[j];
         if (maturity) maturity[j] = sp.mats[j].T;
     }
     return HEXO_OK;

@@ -297,7 +297,7 @@ void cv_schedule(const BatchPlan &bp, uint32_t s, uint32_t j, std::vector<double
         if (last) break;
     }
     const MatDesc &md = bp.mats[sd.mat_begin + j];
-    const double T = md.T, w = md.tmtp / md.dt;
+    const double T = md.T, w = md.w;
     const size_t n = dts.size();
     std::vector<double> c(n, 0.0);
     for (size_t k = 1; k < n; ++k) {

@@ -33,24 +33,11 @@ __device__ __forceinline__ float head(double x) {
 __device__ __forceinline__ float pow2_of(double x) {
     return __uint_as_float(((hi32(x) << 3) & 0x7f800000u) ^ 0x40000000u);
 }
-// A float near a signed x, |x| < 2^128 (24 leading bits; below 2^-126: 0).
-__device__ __forceinline__ float to_float(double x) {
-    const uint32_t h = hi32(x), a = h & 0x7fffffffu;
-    const uint32_t b = a < 0x38100000u ? 0u : (__funnelshift_l(lo32(x), a, 3) & 0x7fffffffu) ^ 0x40000000u;
-    return __uint_as_float(b | (h & 0x80000000u));
-}
 // f as a double: exact for normal f; 0 and subnormals become values below 2^-126.
 __device__ __forceinline__ double to_double(float f) {
     const uint32_t b = __float_as_uint(f);
     return from_words(((uint32_t)((int32_t)b >> 3) & 0x8fffffffu) + 0x38000000u, b << 29);
 }
-// x / 2 for |x| >= 2^-1000, else 0.
-__device__ __forceinline__ double half(double x) {
-    const uint32_t h = hi32(x);
-    const bool tiny = (h & 0x7fffffffu) < 0x01700000u;
-    return from_words(tiny ? 0u : h - 0x00100000u, tiny ? 0u : lo32(x));
-}
-
 // x as a double-single value, 2^-74 <= x < 2^100: head and the other 29 bits.
 __device__ __forceinline__ ds::F2 split(double x) {
     const float h = head(x);
@@ -98,7 +85,7 @@ __device__ __forceinline__ float remainder_sqr(double x, double q) {
 
 // ------------------------------------------------------------------ tables
 //
-// 2^(j/256) and, for the logarithm, 512 reciprocals with their logarithms,
+// 2^(j/256) and, for the logarithm, 512 short reciprocals with their logarithms,
 // computed at compile time in double-double arithmetic (Dekker's splitting
 // and Knuth's TwoSum, as in hexo_ds.cuh) from the exponential and inverse
 // hyperbolic tangent series.
@@ -148,23 +135,27 @@ constexpr DD dd_log_ratio(DD num, DD den) {   // log((den + num) / (den - num)) 
 }
 constexpr DD kLn2 = dd_log_ratio(DD{1.0, 0.0}, DD{3.0, 0.0});
 
-constexpr int kExpTab = 256;   // a CTA's copy in shared memory: kExpTab * 12 bytes
+// A double-double value's x.h + x.l, 0 <= x < 4, in units of 2^-62 (to nearest).
+constexpr uint64_t dd_fixed62(DD x) {
+    const double s = 4611686018427387904.0;                  // 2^62
+    const uint64_t h = (uint64_t)(x.h * s);                  // exact: x.h has 53 bits
+    const double r = x.h * s - (double)h + x.l * s;
+    return h + (uint64_t)(int64_t)(r < 0.0 ? r - 0.5 : r + 0.5);
+}
+
+constexpr int kExpTab = 256;   // a CTA's copy in shared memory: kExpTab * 8 bytes
 struct ExpTab {
-    double t[kExpTab];         // 2^(j/256), rounded
-    float l[kExpTab];          // what rounding left, relative to t
+    uint64_t t[kExpTab];       // 2^(j/256) in units of 2^-62
 };
 constexpr ExpTab make_exp_tab() {
     ExpTab r{};
-    for (int j = 0; j < kExpTab; ++j) {
-        const DD e = dd_exp(dd_mul(kLn2, DD{(double)j / kExpTab, 0.0}));
-        r.t[j] = e.h;
-        r.l[j] = (float)(e.l / e.h);
-    }
+    for (int j = 0; j < kExpTab; ++j) r.t[j] = dd_fixed62(dd_exp(dd_mul(kLn2, DD{(double)j / kExpTab, 0.0})));
     return r;
 }
 constexpr int kLogTab = 512;
 struct LogEntry {
-    double inv, lg;            // 1 / c_j, c_j the middle of the j-th of 512 parts of [1, 2), and -log of it
+    uint64_t lg;               // -log(inv 2^-12) in units of 2^-57
+    uint32_t inv, pad;         // round(2^12 / c_j), c_j the middle of the j-th of 512 parts of [1, 2)
 };
 struct LogTab {
     LogEntry e[kLogTab];
@@ -172,9 +163,9 @@ struct LogTab {
 constexpr LogTab make_log_tab() {
     LogTab r{};
     for (int j = 0; j < kLogTab; ++j) {
-        const double inv = 1.0 / (1.0 + (j + 0.5) / kLogTab);
-        const DD lg = dd_log_ratio(DD{1.0 - inv, 0.0}, dd_two_sum(1.0, inv));
-        r.e[j] = LogEntry{inv, lg.h};
+        const uint32_t inv = (uint32_t)(4096.0 / (1.0 + (j + 0.5) / kLogTab) + 0.5);
+        const DD lg = dd_log_ratio(DD{4096.0 - inv, 0.0}, DD{4096.0 + inv, 0.0});
+        r.e[j] = LogEntry{(dd_fixed62(lg) + 16u) >> 5, inv, 0u};
     }
     return r;
 }
@@ -183,54 +174,65 @@ __device__ constexpr LogTab kLogTabDev = make_log_tab();
 
 // A CTA's copy of the exponential's table, visible after the next barrier.
 __device__ __forceinline__ void exp_table_init(ExpTab *t, uint32_t tid, uint32_t nthreads) {
-    for (uint32_t j = tid; j < (uint32_t)kExpTab; j += nthreads) {
-        t->t[j] = kExpTabInit.t[j];
-        t->l[j] = kExpTabInit.l[j];
-    }
+    for (uint32_t j = tid; j < (uint32_t)kExpTab; j += nthreads) t->t[j] = kExpTabInit.t[j];
 }
 
 // ----------------------------------------------------------- exp, log, root
 
-// exp(x): x = n ln2/256 + r, |r| <= ln2/512, and 2^(n/256) (1 + r + r^2/2 +
-// c) with c = r^3/6 + r^4/24 + r^5/120, below 2^-31, the table's own remainder and n
-// times what ln2/256 lost to rounding, all in float (1/6 rounded up by what
-// to_float's truncation takes from r^3 on average).  Four FP64 instructions
-// (the library's exp takes the time of 18) and an error below 1 ulp.
-__device__ __forceinline__ double exp_tab(double x, const ExpTab *tab) {
-    if (((hi32(x) & 0x7fffffffu) >= 0x40800000u)) return exp(x);   // |x| >= 512, infinite or NaN
-    constexpr double L = kLn2.h / kExpTab;
-    constexpr float Ll = (float)(kLn2.l / kExpTab), invL = (float)(kExpTab / kLn2.h);
-    const float t = __fmaf_rn(to_float(x), invL, 0x1.8p23f);       // rounds to an integer, |n| < 2^18
-    const int n = (int)__float_as_uint(t) - 0x4b400000;
-    const float nf = __fsub_rn(t, 0x1.8p23f);
-    const double r = __fma_rn(-to_double(nf), L, x);
-    const uint32_t j = (uint32_t)n & (uint32_t)(kExpTab - 1);
-    const float rf = to_float(r);
-    const float c3 = __fmul_rn(__fmul_rn(rf, rf), __fmul_rn(rf, __fmaf_rn(rf, __fmaf_rn(rf, 0x1.111112p-7f, 0x1.555556p-5f), 0x1.555558p-3f)));
-    const float c = __fadd_rn(c3, __fmaf_rn(-nf, Ll, tab->l[j]));
-    const double u = __dadd_rn(__fma_rn(r, half(r), r), to_double(c));
-    const double T = tab->t[j];
-    const double Ts = from_words(hi32(T) + ((uint32_t)(n >> 8) << 20), lo32(T));   // T 2^(n >> 8), normal
-    return __fma_rn(Ts, u, Ts);
+__device__ __forceinline__ uint32_t hi(uint64_t x) { return (uint32_t)(x >> 32); }
+__device__ __forceinline__ uint32_t lo(uint64_t x) { return (uint32_t)x; }
+// a b 2^-64, at most 3 too small (the low words' product is left out).
+__device__ __forceinline__ uint64_t mul_hi(uint64_t a, uint64_t b) {
+    return (uint64_t)hi(a) * hi(b) + __umulhi(hi(a), lo(b)) + __umulhi(lo(a), hi(b));
+}
+// r^2 2^64 of r 2^-64, at most 1 too small.
+__device__ __forceinline__ uint64_t sqr_hi(uint64_t r) {
+    return (uint64_t)hi(r) * hi(r) + 2ull * __umulhi(hi(r), lo(r));
 }
 
-// log(x) (1 + d) for 2^-80 < x < 2 and a relative correction |d| < 2^-40 of
-// both x and the result (log(x (1 + d)) (1 + d) to first order): x = 2^k M, M
-// in [1, 2), r = M / c_j - 1, |r| <= 2^-10, log x = k ln2 + log c_j + (r -
-// r^2/2) + c, c = r^3/3 - r^4/4 + r^5/5 below 2^-31 and the corrections in
-// float (1/3 rounded up as 1/6 above).  Five FP64 instructions (the library's
-// log takes the time of 28).
-__device__ __forceinline__ double log_tab(double x, float d) {
-    const uint32_t h = hi32(x);
-    const int k = (int)(h >> 20) - 1023;
-    const LogEntry e = kLogTabDev.e[(h >> 11) & (uint32_t)(kLogTab - 1)];
-    const double r = __fma_rn(from_words((h & 0x000fffffu) | 0x3ff00000u, lo32(x)), e.inv, -1.0);
-    const float kf = (float)k, rf = to_float(r);
-    const float c3 = __fmul_rn(__fmul_rn(rf, rf), __fmul_rn(rf, __fmaf_rn(rf, __fmaf_rn(rf, 0.2f, -0.25f), 0x1.555558p-2f)));
-    const float lf = __logf(head(x));
-    const float c = __fadd_rn(c3, __fmaf_rn(d, __fadd_rn(1.0f, lf), __fmul_rn(kf, (float)kLn2.l)));
-    const double u = __dadd_rn(__fma_rn(r, -half(r), r), to_double(c));
-    return __dadd_rn(__fma_rn(to_double(kf), kLn2.h, e.lg), u);
+// exp(x) in integer arithmetic, within 0.6 ulp: x in units of 2^-54 is n
+// ln2/256 + r, 0 <= r < ln2/256 (1 + 2^-11), r in units of 2^-71, and the
+// result 2^(n/256) (1 + r + r^2/2 + r^3 (1/6 + r/24 + r^2/120)) in units of
+// 2^-62.  No FP64 instruction (the library's exp takes the time of 18).
+__device__ __forceinline__ double exp_tab(double x, const ExpTab *tab) {
+    const uint32_t xh = hi32(x), a = xh & 0x7fffffffu;
+    if (a >= 0x40800000u) return exp(x);   // |x| >= 512, infinite or NaN
+    const uint64_t M = ((uint64_t)((a << 10 & 0x3fffffffu) | 0x40000000u) << 32 | (uint64_t)(lo32(x) >> 22) << 32) |
+                       (uint64_t)(lo32(x) << 10);
+    uint64_t F = M >> min(1031u - (a >> 20), 63u);
+    if ((int32_t)xh < 0) F = 0ull - F;
+    const int32_t n = __mulhi((int32_t)hi(F) - 2, (int32_t)(kExpTab / kLn2.h * 0x1p22)) >> 12;
+    constexpr uint64_t L71 = (uint64_t)(kLn2.h / kExpTab * 0x1p71) + (uint64_t)(int64_t)(kLn2.l / kExpTab * 0x1p71 + 0.5);
+    const uint64_t r = (F << 17) - (uint64_t)(int64_t)n * L71;
+    const uint32_t rh = hi(r);
+    const uint32_t p = 2863311531u + __umulhi(rh, 5592405u + __umulhi(rh, 8738u));   // 1/6 + r/24 + r^2/120, 2^-34
+    const uint32_t q = __umulhi(rh << 1, p) << 1;                                    // r p, 2^-43
+    const uint64_t r2 = sqr_hi(r);                                                   // r^2, 2^-78
+    const uint64_t u = (r >> 7) + (r2 >> 15) + (uint64_t)__umulhi((uint32_t)(r2 >> 29), q) * 16ull;   // 2^-64
+    const uint64_t T = tab->t[n & (kExpTab - 1)];
+    uint64_t y = T + mul_hi(T, u);
+    const uint32_t s = hi(y) >> 31;        // 2^63 or more: the next binade
+    y >>= s;
+    return __longlong_as_double((long long)(((uint64_t)(1022u + (uint32_t)(n >> 8) + s) << 52) + ((y + 512ull) >> 10)));
+}
+
+// -log(x) in units of 2^-57 of x = P 2^(k-63), 2^63 <= P < 2^64, -80 < k < 0,
+// plus what a relative error d of x and of the result puts on it (log(x (1 +
+// d)) (1 + d) to first order, |d| < 2^-40): r = P inv - 1, |r| < 2^-9.6, exact
+// in units of 2^-71, log x = k ln2 + log c_j + r - r^2/2 + r^3/3 - r^4/4 +
+// r^5/5, the last three in float (below 2^-30; 1/3 rounded up by what cutting
+// r to 24 bits takes on average).
+__device__ __forceinline__ uint64_t neg_log_fixed(uint64_t P, int k, float d) {
+    const LogEntry e = kLogTabDev.e[(uint32_t)(P >> 54) & (uint32_t)(kLogTab - 1)];
+    const int64_t r = (int64_t)((P >> 4) * (uint64_t)e.inv);
+    const uint64_t ra = (uint64_t)(r < 0 ? -r : r);
+    const float rf = __fmul_rn(__int2float_rn((int32_t)(r >> 32)), 0x1p-39f);
+    const float c3 = __fmul_rn(__fmul_rn(rf, rf), __fmul_rn(rf, __fmaf_rn(rf, __fmaf_rn(rf, 0.2f, -0.25f), 0x1.555556p-2f)));
+    const float lf = __fmul_rn(0.6931472f, __fadd_rn((float)k, __log2f(__uint_as_float((hi(P) >> 8 & 0x007fffffu) | 0x3f800000u))));
+    const int32_t c = __float2int_rn(__fmul_rn(__fmaf_rn(d, __fadd_rn(1.0f, lf), c3), 0x1p57f));
+    constexpr uint64_t L57 = (uint64_t)(kLn2.h * 0x1p57) + (uint64_t)(int64_t)(kLn2.l * 0x1p57 + 0.5);
+    const uint64_t l = (uint64_t)(int64_t)k * L57 + e.lg + (uint64_t)(r >> 14) - (sqr_hi(ra) >> 22) + (uint64_t)(int64_t)c;
+    return (int64_t)l < 0 ? 0ull - l : 0ull;
 }
 
 // sqrt(x), within 0.51 ulp (x below 2^-120, 0 included, gives a root below
@@ -250,15 +252,15 @@ __device__ __forceinline__ double root(double x) {
     return __longlong_as_double(__double_as_longlong(S) + (long long)k);
 }
 
-// ---------------------------------------------------------------- QE step
-
-// N 2^-64, N > 0, rounded to double.
-__device__ __forceinline__ double u64_2m64(uint64_t N) {
-    const uint32_t lz = (uint32_t)__clzll((long long)N);
-    const uint64_t n = N << lz;
-    const uint64_t m = (n >> 11) + ((n >> 10) & 1ull);   // a carry moves into the exponent
-    return __longlong_as_double((long long)(((uint64_t)(1021u - lz) << 52) + m));
+// x / y from r = 1 / y rounded (0: not given): the product corrected by its
+// remainder, as exact as a division.
+__device__ __forceinline__ double div_by(double x, double y, double r) {
+    if (r == 0.0) return __ddiv_rn(x, y);
+    const double q = __dmul_rn(x, r), c = __fma_rn(__fma_rn(-q, y, x), r, q);
+    return (hi32(q) & 0x7ff00000u) == 0x7ff00000u ? q : c;   // infinite stays infinite
 }
+
+// ---------------------------------------------------------------- QE step
 
 // m within [2^-30, 2^30), s2 within [2^-60, 2^60) and s2 / m^2 above about
 // 2^-40, where the functions below are used: no double-single intermediate
@@ -318,8 +320,8 @@ __device__ __forceinline__ double variance_quadratic(double m, double s2, float 
 // The exponential branch (HSimulation.tpp:70-73) with Y = (s^2 + m^2) /
 // (2 m^2) = 1 / (1 - p) = 1 / (beta m): log((1-p)/(1-U)) / beta = -m Y
 // log(Y (1 - U)), positive exactly when p < U.  Y is one quotient in
-// double-single, its remainder exact; ten FP64 instructions instead of five
-// divisions and a logarithm.
+// double-single, its remainder exact, and the product is taken in integers;
+// two FP64 instructions instead of five divisions and a logarithm.
 __device__ __forceinline__ double variance_exponential(double m, double s2, uint64_t uw) {
     const double mm = __dmul_rn(m, m), W = __fma_rn(m, m, s2);
     const double mm2 = from_words(hi32(mm) + 0x00100000u, lo32(mm));
@@ -331,11 +333,26 @@ __device__ __forceinline__ double variance_exponential(double m, double s2, uint
     const ds::F2 Yf = ds::fast_two_sum(y0, __fmul_rn(e, rm));
     const uint64_t N = 0ull - uw;                                     // 1 - U = N 2^-64 (uw == 0: U = 0 < p)
     if (N == 0ull) return 0.0;
-    const double Y = join(Yf), om = u64_2m64(N);
-    const double x = __dmul_rn(Y, om);
-    if (hi32(x) >= 0x3ff00000u) return 0.0;                           // p >= U
+    const double Y = join(Yf);
+    // x = Y (1 - U) = P 2^(k-63)
+    const uint64_t Ym = (uint64_t)__double_as_longlong(Y) << 11 | 0x8000000000000000ull;
+    const int lz = __clzll((long long)N);
+    uint64_t P = mul_hi(Ym, N << lz);
+    const int s = (int)(~hi(P) >> 31), eY = (int)(hi32(Y) >> 20) - 1023;
+    const int k = eY - lz - s;
+    if (k >= 0) return 0.0;                                           // p >= U
+    P <<= s;
     const float d = __fdividef(__fmul_rn(remainder_mul(W, Y, mm2), rm), y0);
-    return __dmul_rn(__dmul_rn(-m, Y), log_tab(x, d));
+    // m Y (-log x), its significand in 64 bits
+    uint64_t A = neg_log_fixed(P, k, d);
+    if (A == 0ull) return 0.0;
+    const int la = __clzll((long long)A);
+    uint64_t V = mul_hi((uint64_t)__double_as_longlong(m) << 11 | 0x8000000000000000ull, Ym);   // 2^61.99 or more
+    V = mul_hi(V, A << la);
+    const int lv = __clzll((long long)V);
+    V <<= lv;
+    const uint32_t ev = (hi32(m) >> 20) + (uint32_t)(eY + 8 - la - lv);   // the leading bit's exponent
+    return __longlong_as_double((long long)(((uint64_t)(ev - 1u) << 52) + ((V + 1024ull) >> 11)));
 }
 
 // The next variance outside in_range, in the reference's order of operations.

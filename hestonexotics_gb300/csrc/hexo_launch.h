@@ -11,13 +11,12 @@ namespace hexo {
 // Dynamic shared memory of the path kernel: per path two raw slots (16 x u64)
 // and two normal slots (16 x f32); per warp the conversion queue
 // (kWarpScratchBytes) and a 64-option window of 32-bit payoff sums (16-byte
-// aligned); the FP32 form's 128-entry double-single log table (2 KB) or the
-// FP64 form's 256-entry exponential table (3 KB).
-inline size_t paths_smem_bytes(bool f32, uint32_t block, uint32_t ppt) {
+// aligned); the FP32 form's 128-entry double-single log table or the FP64
+// form's 256-entry exponential table (2 KB either way).
+inline size_t paths_smem_bytes(uint32_t block, uint32_t ppt) {
     const size_t rings = (size_t)ppt * 2 * kRngWords * block * (sizeof(uint64_t) + sizeof(float)) +
                          (size_t)(block / 32) * kWarpScratchBytes;
-    return (rings + 15) / 16 * 16 + (size_t)(block / 32) * 64u * kLimbs * sizeof(uint32_t) +
-           (f32 ? 128u * 16u : 256u * 12u);
+    return (rings + 15) / 16 * 16 + (size_t)(block / 32) * 64u * kLimbs * sizeof(uint32_t) + 2048u;
 }
 
 // nullptr when (ppt, unroll) is not instantiated; the control-variate

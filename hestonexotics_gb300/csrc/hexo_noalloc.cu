@@ -92,8 +92,8 @@ hexo_status na_setup(int dev, bool f32, unsigned char **scratch, uint32_t *grid_
         int sms = 0;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
             return HEXO_ERR_CUDA;
+        const size_t smem = paths_smem_bytes(kNaBlock, 1);
         for (int k = 0; k < 2; ++k) {
-            const size_t smem = paths_smem_bytes(k == 1, kNaBlock, 1);
             const void *fn = paths_kernel_ptr(k == 1, 1, 1);
             int nb = 0;
             if (paths_smem_limit(fn, dev) != cudaSuccess ||
@@ -229,10 +229,7 @@ extern "C" hexo_status hexo_price_noalloc(const hexo_params *pp, double S0, cons
                 seg.mat_begin = j;
                 while (j < m && t >= mats[j].T) {
                     MatDesc &md = mats[j];
-                    md.tmtp = md.T - tp;
-                    md.dt = md.T / mat_steps[j];
-                    md.f_w = (float)(md.tmtp / md.dt);
-                    md.f_invT = (float)(1.0 / md.T);
+                    mat_weights(md, md.T - tp, md.T / mat_steps[j]);
                     seg_of_mat[j] = n_segs;
                     ++j;
                 }
@@ -328,7 +325,7 @@ extern "C" hexo_status hexo_price_noalloc(const hexo_params *pp, double S0, cons
     a.n_opts = n_opts;
     const LaunchShape sh{kNaBlock, 1, 1};
     const uint32_t grid = std::max<uint32_t>(1, std::min(slots, n_tiles));
-    if (e == cudaSuccess && n_tiles > 0) e = launch_paths(f32, sh, grid, paths_smem_bytes(f32, kNaBlock, 1), s, a);
+    if (e == cudaSuccess && n_tiles > 0) e = launch_paths(f32, sh, grid, paths_smem_bytes(kNaBlock, 1), s, a);
     double *d_price = reinterpret_cast<double *>(base + kOffPrice);
     double *d_se = reinterpret_cast<double *>(base + kOffSe);
     if (e == cudaSuccess) {

@@ -47,9 +47,9 @@ struct PathVars {
 // bits for the same path.
 
 // One QE step of one path (HSimulation.tpp:52-86), FP64; returns whether it
-// took the quadratic branch.  The FP64 pipe bounds it: about 100 instructions
-// a step as the reference writes it, 20 (quadratic) or 23 (exponential) with
-// the roots, quotients, log and exp of hexo_f64.cuh.
+// took the quadratic branch.  As the reference writes it, a step is about 100
+// FP64 instructions, and that pipe bounds it; with the roots, quotients, log
+// and exp of hexo_f64.cuh it is 15 (quadratic) or 11 (exponential).
 __device__ __forceinline__ bool qe_step(PathVars<false> &pv, const SegDesc &sg, const double &theta, dev::Shishua &g,
                                         dev::RngLane &c, const dev::Ring &r, const dev::WarpScratch &ws,
                                         const f64::ExpTab *etab) {
@@ -371,8 +371,8 @@ __global__ void __launch_bounds__(512) paths_kernel(const KernelArgs a) {
                         interp = __fmul_rn(__fsub_rn(pv[p].X, pv[p].Xp), M.f_w);
                         asian[p] = __fmul_rn(__fadd_rn(pv[p].acc, interp), M.f_invT);
                     } else {                                               // AsianContract.h:30-32
-                        interp = __ddiv_rn(__dmul_rn(__dsub_rn(pv[p].X, pv[p].Xp), M.tmtp), M.dt);
-                        asian[p] = __ddiv_rn(__dadd_rn(pv[p].acc, interp), M.T);
+                        interp = __dmul_rn(__dsub_rn(pv[p].X, pv[p].Xp), M.w);
+                        asian[p] = f64::div_by(__dadd_rn(pv[p].acc, interp), M.T, M.invT);
                     }
                     euro[p] = add_r(pv[p].Xp, interp);                     // VanillaContract.h:28-29
                     geo[p] = (R)0;
@@ -382,9 +382,9 @@ __global__ void __launch_bounds__(512) paths_kernel(const KernelArgs a) {
                                                       M.f_invT);
                             geo[p] = __fmul_rn(S0f, expf(L));
                         } else {
-                            const double L = __ddiv_rn(
-                                __dadd_rn(accg[p], __ddiv_rn(__dmul_rn(__dsub_rn(yc[p], yp[p]), M.tmtp), M.dt)), M.T);
-                            geo[p] = __dmul_rn(S.S0, exp(L));
+                            const double L = f64::div_by(
+                                __dadd_rn(accg[p], __dmul_rn(__dsub_rn(yc[p], yp[p]), M.w)), M.T, M.invT);
+                            geo[p] = __dmul_rn(S.S0, f64::exp_tab(L, etab));
                         }
                     }
                     if (a.dbg_asian != nullptr && active[p]) {

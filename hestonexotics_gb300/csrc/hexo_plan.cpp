@@ -100,6 +100,7 @@ hexo_status plan_set(const hexo_params &p, double S0, const hexo_option *opts, u
     // step reaches, then continue with the next maturity's width.
     out.seg_of_mat.assign(m, 0);
     out.steps_to_mat.assign(m, 0);
+    out.mat_tmtp.assign(m, 0.0);
     const double sig2 = p.sigma * p.sigma;
     auto make_seg = [&](double dt) {
         SegDesc s{};
@@ -138,10 +139,8 @@ hexo_status plan_set(const hexo_params &p, double S0, const hexo_option *opts, u
             seg.mat_begin = (uint32_t)j;
             while (j < m && t >= T[j]) {
                 MatDesc &md = out.mats[j];
-                md.tmtp = T[j] - tp;
-                md.dt = T[j] / out.mat_steps[j];
-                md.f_w = (float)(md.tmtp / md.dt);
-                md.f_invT = (float)(1.0 / T[j]);
+                out.mat_tmtp[j] = T[j] - tp;
+                mat_weights(md, out.mat_tmtp[j], T[j] / out.mat_steps[j]);
                 out.seg_of_mat[j] = (uint32_t)out.segs.size();
                 out.steps_to_mat[j] = steps_total;
                 ++j;

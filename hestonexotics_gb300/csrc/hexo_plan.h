@@ -24,6 +24,7 @@ struct SetPlan {
     std::vector<OptDesc> opts;          // sorted by maturity; out_index = request-local option index
     std::vector<double> opt_disc;       // exp(-r T) per sorted option
     std::vector<uint32_t> mat_steps;    // nominal steps per maturity
+    std::vector<double> mat_tmtp;       // T - t_prev of the step that prices the maturity
     std::vector<uint64_t> mat_paths;    // max paths over the maturity's options
     std::vector<uint64_t> thr;          // thr[j] = max_{j' >= j} mat_paths[j'] (paths that reach maturity j)
     std::vector<uint32_t> seg_of_mat;   // segment whose last step prices maturity j

@@ -68,7 +68,7 @@ extern "C" hexo_status hexo_autotune(hexo_ctx *ctx, const hexo_request *reqs, ui
                 size_t smem;
                 uint32_t ctas;
                 const LaunchShape sh{b, p, u};
-                if (paths_smem_bytes(f32, b, p) > ctx->smem_optin) continue;
+                if (paths_smem_bytes(b, p) > ctx->smem_optin) continue;
                 if (shape_check(ctx, f32, sh, smem, ctas) != HEXO_OK) continue;
                 BatchPlan bp;
                 std::vector<SetPlan> plans;

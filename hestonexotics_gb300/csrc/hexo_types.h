@@ -70,9 +70,9 @@ struct SegDesc {
 
 struct MatDesc {
     double T;       // maturity
-    double tmtp;    // T - t_prev of the pricing step (AsianContract.h:30-31)
-    double dt;      // T / steps at pricing time (the contract's init_step_size)
-    float f_w;      // tmtp / dt
+    double w;       // (T - t_prev) / dt of the pricing step (AsianContract.h:30-31)
+    double invT;    // 1 / T, or 0 for a T whose reciprocal could leave the double range
+    float f_w;      // w
     float f_invT;   // 1 / T
     uint32_t opt_begin, opt_end;   // set-local option range (options sorted by maturity)
 };
@@ -111,6 +111,14 @@ struct TileDesc {
 inline void ds_split(double x, float out[2]) {
     out[0] = (float)x;
     out[1] = (float)(x - (double)out[0]);
+}
+
+// w = (T - t_prev) / dt, dt = T / steps the contract's init_step_size, and 1 / T
+inline void mat_weights(MatDesc &m, double tmtp, double dt) {
+    m.w = tmtp / dt;
+    m.invT = m.T > 0x1p-500 && m.T < 0x1p500 ? 1.0 / m.T : 0.0;
+    m.f_w = (float)m.w;
+    m.f_invT = (float)(1.0 / m.T);
 }
 
 struct KernelArgs {
