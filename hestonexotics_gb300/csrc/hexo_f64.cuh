@@ -252,6 +252,17 @@ __device__ __forceinline__ double root(double x) {
     return __longlong_as_double(__double_as_longlong(S) + (long long)k);
 }
 
+// 1 / x within 0.51 ulp, 2^-60 < x < 2^60, like root without an FP64 instruction.
+__device__ __forceinline__ double recip(double x) {
+    const ds::F2 xs = split(x);
+    const float r = ds::rcp_approx(xs.h);
+    const ds::F2 y = ds::fast_two_sum(r, __fmul_rn(__fmaf_rn(-r, xs.l, __fmaf_rn(-r, xs.h, 1.0f)), r));
+    const double Y = join(y);
+    const float unit = __uint_as_float(0x7f000000u + (52u << 23) - (__float_as_uint(y.h) & 0x7f800000u));
+    const int32_t k = __float2int_rn(__fmul_rn(__fmul_rn(remainder_mul(1.0, x, Y), r), unit));
+    return __longlong_as_double(__double_as_longlong(Y) + (long long)k);
+}
+
 // x / y from r = 1 / y rounded (0: not given): the product corrected by its
 // remainder, as exact as a division.
 __device__ __forceinline__ double div_by(double x, double y, double r) {

@@ -13,10 +13,10 @@
 //   c_j  = sum_k V_k w^{k(2j+1)} sqrt(2^m) / J                      (SWIFT.cpp:69-72)
 //   price_i (and gradient) = Re sum_j phi(u_j) c_j disc K_i e^{-i u_j x_i}  (SWIFT.cpp:102-118)
 // with w = e^{i pi / (2J)} and x_i = r tau + log(S / K_i).  The reference
-// evaluates the two transforms with FFTW; here they are direct sums (the same
-// sums), spread one warp per 32 outputs over the whole GPU.  Everything is
-// FP64: the work per call is small and the results must match the
-// reference's known answers to 1e-9.
+// evaluates the two transforms with FFTW; here they are FFTs in shared memory
+// (fft_part), or the direct sums where the caller asks for them or J is tiny.  Everything is FP64, since the results must match the reference's
+// known answers to 1e-9, and the FP64 pipe (2 lanes per cycle and SM) bounds
+// every kernel.
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cmath>
@@ -27,6 +27,7 @@
 
 #include "hexo_mc.h"
 #include "hexo_runtime.h"
+#include "hexo_f64.cuh"
 
 namespace hexo {
 namespace swift {
@@ -116,8 +117,9 @@ __host__ __device__ inline cplx chf(const HP &p, double tau, cplx u, const Aux &
     return cexp_((p.kappa * p.vm * p.rho * tau) * (u * I) / p.sigma - a.A + (2.0 * p.kappa * p.vm) * a.D / (p.sigma * p.sigma));
 }
 
-// phi and its partial derivatives in (v0, vm, rho, kappa, sigma) (HDistribution.cpp:48-84)
-__host__ __device__ inline void chf_grad(const HP &p, double tau, cplx u, cplx out[6]) {
+// phi and its partial derivatives in (v0, vm, rho, kappa, sigma), in the
+// reference's order of operations (HDistribution.cpp:48-84).
+__host__ __device__ inline void chf_grad_reference(const HP &p, double tau, cplx u, cplx out[6]) {
     const cplx I = C(0.0, 1.0);
     const Aux a = aux(p, u, tau);
     const cplx c = chf(p, tau, u, a);
@@ -148,6 +150,82 @@ __host__ __device__ inline void chf_grad(const HP &p, double tau, cplx u, cplx o
     out[3] = c * g_rho;
     out[4] = c * g_kappa;
     out[5] = c * g_sigma;
+}
+
+// phi and its partial derivatives in (v0, vm, rho, kappa, sigma) at a real
+// frequency u (HDistribution.cpp:48-84).  The reference's A1, A2 and B hold
+// sinh and cosh of d tau / 2; here both are taken out as T = tanh(d tau / 2),
+// so A2 = cosh Q / v0 with Q = d + xi T, every logarithmic derivative is a
+// polynomial in f, xi, d, T and the two reciprocals 1/d and 1/Q:
+//   A = v0 f T / Q, D = log(2 d / ((1 + E) Q)) + (kappa - d) tau / 2, E = e^{-d tau},
+//   a2r = A2_rho / A2 = W (2 + xi tau) (xi + d T) / (2 d Q),  W = i sigma u,
+//   A_rho = fv d_rho - A a2r,  fv = v0 tau f / (2 Q),  d_rho = xi W / d, and so on.
+// T = (1 - |E|^2 - 2 i Im E) / |1 + E|^2 from expm1 keeps its accuracy for
+// small d tau.  One exp, one expm1, two sincos, one log, one atan2 and about
+// 45 complex products: some 350 FP64 instructions, against 1,400 with the
+// two dozen complex quotients of the reference's form.  False, for that form,
+// from d tau / 2 = 300 on, where sinh, cosh and the squares of A2 come near the
+// end of the double range: what it gives there (phi is below e^{-300}, and
+// beyond the range the result is NaN) is what it gave before.
+__device__ __forceinline__ double recip(double x) {   // 1 / x, x > 0
+    return x > 0x1p-60 && x < 0x1p60 ? f64::recip(x) : 1.0 / x;
+}
+__device__ __forceinline__ double sqroot(double x) {   // sqrt(x), x >= 0
+    return x > 0x1p-100 && x < 0x1p100 ? f64::root(x) : sqrt(x);
+}
+__device__ __forceinline__ double norm(cplx a) { return a.re * a.re + a.im * a.im; }
+__device__ __forceinline__ cplx conj(cplx a) { return C(a.re, -a.im); }
+
+struct ChfConst {   // of one expiry
+    double is, k2, rs;   // 1 / sigma, 2 kappa vm / sigma^2, rho / sigma
+};
+
+__device__ __forceinline__ bool chf_grad(const HP &p, const ChfConst &q, double tau, double u, cplx out[6]) {
+    const double su = p.sigma * u;
+    const cplx xi = C(p.kappa, su * p.rho), f = C(u * u, -u);
+    // d = sqrt(xi^2 + sigma^2 f), principal
+    const cplx d2 = C(xi.re * xi.re - xi.im * xi.im + su * su, 2.0 * xi.re * xi.im - p.sigma * su);
+    const double r = sqroot(norm(d2)), t0 = sqroot(0.5 * (r + fabs(d2.re))), t1 = 0.5 * fabs(d2.im) * recip(t0);
+    const cplx d = C(d2.re >= 0.0 ? t0 : t1, copysign(d2.re >= 0.0 ? t1 : t0, d2.im));
+    if (!(d.re * tau < 600.0) || p.v0 < 1e-12) return false;
+    double sn, cs;
+    sincos(d.im * tau, &sn, &cs);
+    const double em = expm1(-(d.re * tau)), a = 1.0 + em;   // E = a (cs - i sn)
+    const double iden = recip(1.0 + a * (2.0 * cs + a));    // 1 / |1 + E|^2
+    const cplx T = C(-em * (2.0 + em) * iden, 2.0 * a * sn * iden);
+    const cplx Q = d + xi * T;
+    const cplx iQ = conj(Q) * recip(norm(Q)), id = conj(d) * recip(norm(d));
+    const cplx fq = f * iQ, A = p.v0 * (fq * T);
+    const cplx z = (2.0 * iden) * (d * C(1.0 + a * cs, a * sn)) * iQ;
+    const cplx D = C(0.5 * log(norm(z)) + (p.kappa - d.re) * (0.5 * tau), atan2(z.im, z.re) - d.im * (0.5 * tau));
+    const double vt = p.vm * tau * u * q.is;   // t = vm tau i u / sigma
+    const double er = q.k2 * D.re - A.re, ei = p.kappa * p.rho * vt + q.k2 * D.im - A.im;
+    double ps, pc;
+    sincos(ei, &ps, &pc);
+    const double ea = f64::exp_tab(er, &f64::kExpTabInit);
+    const cplx c = C(ea * pc, ea * ps);
+    const cplx W = C(0.0, su), h = C(2.0 + xi.re * tau, xi.im * tau);
+    const cplx xw = xi * W, d_rho = xw * id;
+    const cplx a2r = (0.5 * (W * h)) * ((xi + d * T) * (id * iQ));
+    const cplx fv = (0.5 * tau * p.v0) * fq;
+    const cplx A_rho = fv * d_rho - A * a2r;
+    const cplx br = d_rho * id - a2r;                        // B_rho / B
+    const cplx d_sigma = (q.rs * xw - W + su * u) * id;
+    const cplx a2s = q.rs * a2r + (0.5 * p.sigma) * (fq * (h * id + tau * T));
+    const cplx A_sigma = fv * d_sigma - A * a2s;
+    const double iw = -q.is / u;                              // 1 / W = i iw
+    const cplx i_br = C(-iw * br.im, iw * br.re), i_ar = C(-iw * A_rho.im, iw * A_rho.re);
+    out[0] = c;
+    out[1] = -(c * (fq * T));
+    out[2] = c * ((2.0 * p.kappa * q.is * q.is) * D + C(0.0, p.kappa * p.rho * tau * u * q.is));
+    out[3] = c * (q.k2 * br - A_rho + C(0.0, vt * p.kappa));
+    out[4] = c * (q.k2 * (i_br + 0.5 * tau) - i_ar + (2.0 * p.vm * q.is * q.is) * D + C(0.0, vt * p.rho));
+    out[5] = c * (q.k2 * (d_sigma * id - a2s) - A_sigma - (2.0 * q.k2 * q.is) * D - C(0.0, vt * p.rho * p.kappa * q.is));
+    return true;
+}
+
+static __device__ __noinline__ void chf_grad_far(const HP &p, double tau, double u, cplx out[6]) {
+    chf_grad_reference(p, tau, C(u), out);
 }
 
 // ------------------------------------------------ dynamic wavelet parameters
@@ -195,35 +273,68 @@ double cum4(const HP &p, double t) {
 // ------------------------------------------------------------------ kernels
 
 constexpr uint32_t kMaxJ = 1u << 16;
+constexpr int kLogParts = 3, kLogMaxPart = 13;   // parts of an FFT, and the points of one (128 KB) at most
 
 struct Exp {                 // one expiry of one request
     HP p;
+    ChfConst q;
     double tau, r, S, sqrt2m, lower, upper, du;   // du = pi 2^m / (2J): u_j = (2j + 1) du
     int32_t k1, k2;
     uint32_t J, n_opt;
     uint64_t tw_off, h_off, v_off, w_off, o_off;  // element offsets into the work buffers
-    uint32_t fft, logN;      // the two transforms by FFT of length N = 2J = 2^logN (else direct sums)
-    uint64_t f_off;          // its two N-element FFT buffers in the FFT workspace
+    uint32_t logN, logR;     // N = 2J in R parts (the transforms by FFT), or logN = 0: direct sums
+    uint64_t y_off;          // its N results of a transform's parts
+    uint32_t stiff, pad;     // see kStiff
 };
 
-// Expiries with at least this many frequencies use the FFT (automatic method).
-constexpr uint32_t kFftMinJ = 1024;
+// Expiries with fewer frequencies than this use the direct sums (automatic
+// method).
+constexpr uint32_t kFftMinJ = 16, kFftMinStiffJ = 1024;
 
-struct Item {                // 32 consecutive outputs of one expiry
+// An expiry whose range of log prices ends above this is stiff: its payoff
+// terms grow as e^upper and cancel to a price of order K, so the last bits of
+// every factor reach the result e^upper times larger.  Any change of rounding
+// there moves prices by 1e-9 relative at upper = 17 and 1e-7 at 25 (long
+// maturities at high vol-of-vol; measured), below the line by less than 1e-11.
+// Stiff expiries keep the reference's order of operations throughout, so that
+// their results do not move: its characteristic function, a sincos for every
+// phase, and the direct sums below kFftMinStiffJ frequencies.
+constexpr double kStiff = 12.0;
+
+struct Item {                // a block's piece of one expiry: outputs from first on, or an FFT part
     uint32_t e, first;
 };
 
-// w^n = e^{i pi n / (2J)} for n < 4J, and the payoff terms h_j.
-__global__ void tables_kernel(const Exp *ex, const Item *items, uint32_t n_items, double2 *tw, double2 *h) {
-    const uint32_t it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (it >= n_items) return;
-    const Exp E = ex[items[it].e];
-    const uint32_t n = items[it].first + (threadIdx.x & 31u);
-    if (n >= 4 * E.J) return;
-    double s, c;
-    sincospi((double)n / (double)(2 * E.J), &s, &c);
-    tw[E.tw_off + n] = make_double2(c, s);
-    if (n < E.J) {
+struct TwiddleAt {
+    uint64_t off[17];        // element offset of the table of J = 2^i frequencies
+};
+
+// What an option needs of its strike: x, disc K, and its phase's turn over 32 frequencies.
+struct Opt {
+    double x, f, ts, tc;
+};
+
+// The tables of a call in one launch, n_tw + n_h + n_o blocks of 128 threads:
+// w^n = e^{i pi n / (2J)} for n < 4J, one table per distinct J (items: log2 J,
+// first n); the payoff terms h_j, one thread per j; and the options' terms,
+// one thread per option (a warp each in price_kernel would spend as many FP64
+// instructions on them as on a third of its sum).
+__global__ void __launch_bounds__(128) setup_kernel(const Exp *ex, const Item *items, uint32_t n_tw, uint32_t n_h,
+                                                    const TwiddleAt at, const double *strikes, double2 *tw, double2 *h,
+                                                    Opt *opts) {
+    const Item it = items[blockIdx.x];
+    const uint32_t n = it.first + threadIdx.x;
+    if (blockIdx.x < n_tw) {
+        const uint32_t J = 1u << it.e;
+        if (n >= 4 * J) return;
+        double s, c;
+        sincospi((double)n / (double)(2 * J), &s, &c);
+        tw[at.off[it.e] + n] = make_double2(c, s);
+        return;
+    }
+    const Exp &E = ex[it.e];
+    if (blockIdx.x < n_tw + n_h) {
+        if (n >= E.J) return;
         const double u = (2.0 * n + 1.0) * E.du;
         auto H = [&](double y, double ey) {     // -i e^{-i u y} (1/u - ey/(i + u))
             double sy, cy;
@@ -235,94 +346,162 @@ __global__ void tables_kernel(const Exp *ex, const Item *items, uint32_t n_items
         const double lo = fmax(E.lower, 0.0);
         const cplx v = H(E.upper, exp(E.upper)) - H(lo, exp(lo));
         h[E.h_off + n] = make_double2(v.re, v.im);
+        return;
     }
+    if (n >= E.n_opt) return;
+    const double K = strikes[E.o_off + n];
+    Opt o;
+    o.x = E.r * E.tau + log(E.S / K);
+    o.f = exp(-E.r * E.tau) * K;
+    sincos(64.0 * E.du * o.x, &o.ts, &o.tc);
+    opts[E.o_off + n] = o;
 }
 
-// ------------------------------------------------------------------- FFT
+// ------------------------------------------------------------- transforms
 //
 // Both transforms are inverse DFTs of length N = 2J: with w = e^{i pi/(2J)},
 // w^{k(2j+1)} = w^k e^{2 pi i k j / N}, so
 //   V_k = Re(w^k F[k mod N]) sqrt(2^m)/J,  F = IDFT_N(h_0 .. h_{J-1}, 0 .. 0),
 //   c_j = w^{2 k1 j} G[j] sqrt(2^m)/J,     G = IDFT_N(g folded mod N),
-//         g_m = V_{k1+m} w^{k1+m},  m in [0, k2 - k1],
-// IDFT_N(x)[n] = sum_r x_r e^{2 pi i r n / N}.  The IDFT is the radix-2
-// Stockham autosort formulation (Govindaraju et al., "High performance
-// discrete Fourier transforms on graphics processors", SC 2008): log2 N
-// passes, each a butterfly over elements j and j + N/2 whose results land
-// at ((j - k) << 1) + k and that plus Ns, k = j mod Ns, Ns = 2^pass, with
-// twiddle e^{i pi k / Ns}; buffers alternate and the output is in natural
-// order.  O(N log N) instead of the direct sums' O(J (k2 - k1)).
-
-// buffer 0 of an FFT expiry: h_j for j < J, then zeros
-__global__ void fft_load_h_kernel(const Exp *ex, const Item *items, uint32_t n_items, const double2 *h,
-                                  double2 *fbuf) {
-    const uint32_t it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (it >= n_items) return;
-    const Exp E = ex[items[it].e];
-    const uint32_t m = items[it].first + (threadIdx.x & 31u);
-    if (m >= 2 * E.J) return;
-    fbuf[E.f_off + m] = m < E.J ? h[E.h_off + m] : make_double2(0.0, 0.0);
+//         g_m = V_{k1+m} w^{k1+m},  m in [0, k2 - k1].
+// The IDFT is the radix-2 decimation in time of Cooley and Tukey (1965), in R
+// parts: part r runs the n = N / R points r, r + R, ... through log2 n passes
+// in shared memory (fft_terms_kernel for F, fft_payoff_kernel for G, a block
+// each), and the log2 R passes that join the parts run in the registers of
+// whoever reads them: all R outputs q, q + n, ... of a point when the next
+// transform loads its part (they are one residue mod R, the part's own input),
+// one output in density_kernel.  The parts spread an expiry over R SMs, since
+// the FP64 pipe is 2 lanes per cycle and SM; 16 J log2 N FP64 instructions
+// take the place of the direct sums' 4 J (k2 - k1), and two launches that of
+// two per pass.
+__device__ __forceinline__ double2 cmul(double2 a, double2 w) {
+    return make_double2(fma(a.x, w.x, -(a.y * w.y)), fma(a.x, w.y, a.y * w.x));
 }
 
-// buffer 0 of an FFT expiry: the terms V_{k1+m} w^{k1+m} folded mod N
-__global__ void fft_load_g_kernel(const Exp *ex, const Item *items, uint32_t n_items, const double2 *tw,
-                                  const double *V, double2 *fbuf) {
-    const uint32_t it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (it >= n_items) return;
-    const Exp E = ex[items[it].e];
-    const uint32_t r = items[it].first + (threadIdx.x & 31u), N = 2 * E.J;
-    if (r >= N) return;
-    const uint32_t mask = 4 * E.J - 1, K = (uint32_t)(E.k2 - E.k1 + 1);
-    double re = 0.0, im = 0.0;
-    for (uint32_t m = r; m < K; m += N) {   // K <= 4J = 2N: at most two terms
-        const double v = V[E.v_off + m];
-        const double2 t = tw[E.tw_off + ((uint32_t)(E.k1 + (int32_t)m) & mask)];
-        re = fma(v, t.x, re);
-        im = fma(v, t.y, im);
+// A part's passes over n = 2^ln points, in bit-reversed order on entry.
+__device__ __forceinline__ void fft_part(double2 *s, uint32_t ln, const double2 *T, uint32_t J) {
+    for (uint32_t p = 0; p < ln; ++p) {
+        __syncthreads();
+        const uint32_t Ns = 1u << p;
+        for (uint32_t b = threadIdx.x; b < (1u << ln) / 2; b += blockDim.x) {
+            const uint32_t k = b & (Ns - 1u), i = ((b - k) << 1) + k;
+            const double2 x = s[i], z = cmul(s[i + Ns], T[k * ((2u * J) >> p)]);   // e^{i pi k / Ns}
+            s[i] = make_double2(x.x + z.x, x.y + z.y);
+            s[i + Ns] = make_double2(x.x - z.x, x.y - z.y);
+        }
     }
-    fbuf[E.f_off + r] = make_double2(re, im);
+    __syncthreads();
+}
+__device__ __forceinline__ uint32_t bit_reverse(uint32_t i, uint32_t ln) { return ln ? __brev(i) >> (32u - ln) : 0u; }
+
+// y_r of F's part r: the points h_{r + R l}.
+__global__ void __launch_bounds__(128) fft_terms_kernel(const Exp *ex, const Item *items, const double2 *tw,
+                                                        const double2 *h, double2 *y) {
+    extern __shared__ double2 s[];
+    const Exp &E = ex[items[blockIdx.x].e];
+    const uint32_t r = items[blockIdx.x].first, J = E.J, ln = E.logN - E.logR, n = 1u << ln;
+    for (uint32_t l = threadIdx.x; l < n; l += blockDim.x) {
+        const uint32_t j = (l << E.logR) + r;
+        s[bit_reverse(l, ln)] = j < J ? h[E.h_off + j] : make_double2(0.0, 0.0);
+    }
+    fft_part(s, ln, tw + E.tw_off, J);
+    for (uint32_t l = threadIdx.x; l < n; l += blockDim.x) y[E.y_off + r * n + l] = s[l];
 }
 
-// one Stockham pass (Ns = 2^pass) of every FFT expiry with more passes to go
-__global__ void fft_pass_kernel(const Exp *ex, const Item *items, uint32_t n_items, uint32_t pass, double2 *fbuf) {
-    const uint32_t it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (it >= n_items) return;
-    const Exp E = ex[items[it].e];
-    if (pass >= E.logN) return;
-    const uint32_t N = 2 * E.J, half = E.J, j = items[it].first + (threadIdx.x & 31u);
-    if (j >= half) return;
-    const double2 *in = fbuf + E.f_off + (pass & 1u ? N : 0u);
-    double2 *out = fbuf + E.f_off + (pass & 1u ? 0u : N);
-    const uint32_t Ns = 1u << pass, k = j & (Ns - 1u);
-    double s, c;
-    sincospi((double)k / (double)Ns, &s, &c);
-    const double2 a = in[j], b0 = in[j + half];
-    const double2 b = make_double2(b0.x * c - b0.y * s, b0.x * s + b0.y * c);
-    const uint32_t o = ((j - k) << 1) + k;
-    out[o] = make_double2(a.x + b.x, a.y + b.y);
-    out[o + Ns] = make_double2(a.x - b.x, a.y - b.y);
+// F[q + c n], c < R, from the parts' y[q].
+template <int LR>
+__device__ __forceinline__ void fft_join(const double2 *y, uint32_t q, uint32_t ln, const double2 *T, uint32_t J,
+                                         double2 (&v)[1 << LR]) {
+    constexpr int R = 1 << LR;
+    const uint32_t n = 1u << ln;
+#pragma unroll
+    for (int b = 0; b < R; ++b) v[b] = y[(uint32_t)b * n + q];
+#pragma unroll
+    for (int p = 0; p < LR; ++p) {   // v[b 2^p + c]: part b of R / 2^p at q + c n
+        double2 t[R];
+        const int w = 1 << p, half = R >> (p + 1);
+#pragma unroll
+        for (int b = 0; b < half; ++b)
+#pragma unroll
+            for (int c = 0; c < w; ++c) {
+                const double2 x = v[b * w + c];
+                const double2 z = cmul(v[(b + half) * w + c], T[(q + (uint32_t)c * n) * ((2u * J) >> (ln + (uint32_t)p))]);
+                t[b * 2 * w + c] = make_double2(x.x + z.x, x.y + z.y);
+                t[b * 2 * w + c + w] = make_double2(x.x - z.x, x.y - z.y);
+            }
+#pragma unroll
+        for (int b = 0; b < R; ++b) v[b] = t[b];
+    }
 }
 
-// the result of an FFT expiry's transform (after logN passes)
-__device__ __forceinline__ const double2 *fft_result(const Exp &E, const double2 *fbuf) {
-    return fbuf + E.f_off + (E.logN & 1u ? 2u * E.J : 0u);
+// z_r of G's part r: the points g_m, m = r + R l, from F at k1 + m (mod N).
+template <int LR>
+__device__ __forceinline__ void load_payoffs(const Exp &E, uint32_t r, double2 *s, const double2 *T, const double2 *y) {
+    constexpr uint32_t R = 1u << LR;
+    const uint32_t J = E.J, ln = E.logN - (uint32_t)LR, n = 1u << ln, N = 2 * J, mask = 4 * J - 1;
+    const uint32_t K = (uint32_t)(E.k2 - E.k1) + 1u;
+    for (uint32_t q = ((r + (uint32_t)E.k1) & (R - 1u)) + (threadIdx.x << LR); q < n; q += blockDim.x << LR) {
+        double2 f[1 << LR];
+        fft_join<LR>(y, q, ln, T, J, f);
+#pragma unroll
+        for (uint32_t c = 0; c < R; ++c) {
+            const uint32_t m = (q + c * n - (uint32_t)E.k1) & (N - 1u);
+            double re = 0.0, im = 0.0;
+            if (m < K) {
+                const double2 t = T[((uint32_t)E.k1 + m) & mask];
+                const double v = fma(f[c].x, t.x, -f[c].y * t.y) * E.sqrt2m / (double)J;
+                re = fma(v, t.x, re);
+                im = fma(v, t.y, im);
+                if (m + N < K) {   // V_{k+N} = -V_k and w^{k+N} = -w^k: the same term again
+                    re = fma(v, t.x, re);
+                    im = fma(v, t.y, im);
+                }
+            }
+            s[bit_reverse(m >> LR, ln)] = make_double2(re, im);
+        }
+    }
+}
+__global__ void __launch_bounds__(128) fft_payoff_kernel(const Exp *ex, const Item *items, const double2 *tw,
+                                                         const double2 *y, double2 *z) {
+    extern __shared__ double2 s[];
+    const Exp &E = ex[items[blockIdx.x].e];
+    const uint32_t r = items[blockIdx.x].first, ln = E.logN - E.logR, n = 1u << ln;
+    const double2 *T = tw + E.tw_off, *Y = y + E.y_off;
+    if (E.logR == kLogParts) load_payoffs<kLogParts>(E, r, s, T, Y);
+    else if (E.logR == kLogParts + 1) load_payoffs<kLogParts + 1>(E, r, s, T, Y);
+    else load_payoffs<0>(E, r, s, T, Y);
+    fft_part(s, ln, T, E.J);
+    for (uint32_t l = threadIdx.x; l < n; l += blockDim.x) z[E.y_off + r * n + l] = s[l];
 }
 
-// V_k, one lane per k
-__global__ void payoff_kernel(const Exp *ex, const Item *items, uint32_t n_items, const double2 *tw,
-                              const double2 *h, double *V, const double2 *fbuf) {
-    const uint32_t it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (it >= n_items) return;
-    const Exp E = ex[items[it].e];
-    const int32_t k = E.k1 + (int32_t)(items[it].first + (threadIdx.x & 31u));
+// G[j] from its parts.
+template <int LR>
+__device__ __forceinline__ double2 fft_output(const double2 *z, uint32_t j, uint32_t ln, const double2 *T, uint32_t J) {
+    constexpr int R = 1 << LR;
+    double2 v[R];
+#pragma unroll
+    for (int b = 0; b < R; ++b) v[b] = z[((uint32_t)b << ln) + (j & ((1u << ln) - 1u))];
+#pragma unroll
+    for (int p = 0; p < LR; ++p) {
+        const uint32_t Ns = 1u << (ln + (uint32_t)p);
+        const double2 w = T[(j & (Ns - 1u)) * ((2u * J) >> (ln + (uint32_t)p))];
+        const bool up = (j & Ns) != 0u;
+#pragma unroll
+        for (int b = 0; b < (R >> (p + 1)); ++b) {
+            const double2 x = v[b], t = cmul(v[b + (R >> (p + 1))], w);
+            v[b] = up ? make_double2(x.x - t.x, x.y - t.y) : make_double2(x.x + t.x, x.y + t.y);
+        }
+    }
+    return v[0];
+}
+
+// V_k by the direct sum, one lane per k
+__global__ void payoff_kernel(const Exp *ex, const Item *items, const double2 *tw, const double2 *h, double *V) {
+    const Exp &E = ex[items[blockIdx.x].e];
+    const int32_t k = E.k1 + (int32_t)(items[blockIdx.x].first + threadIdx.x);
     if (k > E.k2) return;
     const uint32_t mask = 4 * E.J - 1;
     const double2 *T = tw + E.tw_off;
-    if (E.fft) {   // Re(w^k F[k mod N])
-        const double2 f = fft_result(E, fbuf)[(uint32_t)k & (2 * E.J - 1)], t = T[(uint32_t)k & mask];
-        V[E.v_off + (uint32_t)(k - E.k1)] = fma(f.x, t.x, -f.y * t.y) * E.sqrt2m / (double)E.J;
-        return;
-    }
     const double2 *Hh = h + E.h_off;
     double acc = 0.0;
     uint32_t idx = (uint32_t)k & mask, step = ((uint32_t)(2 * k)) & mask;   // k (2j + 1) mod 4J
@@ -334,20 +513,26 @@ __global__ void payoff_kernel(const Exp *ex, const Item *items, uint32_t n_items
     V[E.v_off + (uint32_t)(k - E.k1)] = acc * E.sqrt2m / (double)E.J;
 }
 
-// c_j and phi(u_j) c_j with its gradient, one lane per j
-__global__ void density_kernel(const Exp *ex, const Item *items, uint32_t n_items, const double2 *tw,
-                               const double *V, double2 *W, const double2 *fbuf) {
-    const uint32_t it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (it >= n_items) return;
-    const Exp E = ex[items[it].e];
-    const uint32_t j = items[it].first + (threadIdx.x & 31u);
+// c_j and phi(u_j) c_j with its gradient, one lane per j; a kernel of its own
+// for stiff expiries (kStiffForm), so that the reference's expressions are
+// compiled by themselves and round as they always did.
+template <bool kStiffForm>
+__global__ void __launch_bounds__(64) density_kernel(const Exp *ex, const Item *items, const double2 *tw,
+                                                     const double *V, double2 *W, const double2 *z) {
+    const Exp E = ex[items[blockIdx.x].e];   // a copy: the stiff form's contractions depend on it
+    const uint32_t j = items[blockIdx.x].first + threadIdx.x;
     if (j >= E.J) return;
     const uint32_t mask = 4 * E.J - 1;
     const double2 *T = tw + E.tw_off;
     const uint32_t odd = 2 * j + 1;
     double re = 0.0, im = 0.0;
-    if (E.fft) {   // w^{2 k1 j} G[j]
-        const double2 g = fft_result(E, fbuf)[j], t = T[((uint32_t)E.k1 * 2u * j) & mask];
+    if (E.logN) {   // w^{2 k1 j} G[j]
+        const double2 *Z = z + E.y_off;
+        const uint32_t ln = E.logN - E.logR;
+        const double2 g = E.logR == kLogParts ? fft_output<kLogParts>(Z, j, ln, T, E.J)
+                          : E.logR == kLogParts + 1 ? fft_output<kLogParts + 1>(Z, j, ln, T, E.J)
+                                                    : fft_output<0>(Z, j, ln, T, E.J);
+        const double2 t = T[((uint32_t)E.k1 * 2u * j) & mask];
         re = fma(g.x, t.x, -g.y * t.y);
         im = fma(g.x, t.y, g.y * t.x);
     } else {
@@ -364,7 +549,8 @@ __global__ void density_kernel(const Exp *ex, const Item *items, uint32_t n_item
     const double sc = E.sqrt2m / (double)E.J;
     const cplx c = C(re * sc, im * sc);
     cplx g[6];
-    chf_grad(E.p, E.tau, C((double)odd * E.du), g);
+    if constexpr (kStiffForm) chf_grad_reference(E.p, E.tau, C((double)odd * E.du), g);
+    else if (!chf_grad(E.p, E.q, E.tau, (double)odd * E.du, g)) chf_grad_far(E.p, E.tau, (double)odd * E.du, g);
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
         const cplx w = g[q] * c;
@@ -372,34 +558,58 @@ __global__ void density_kernel(const Exp *ex, const Item *items, uint32_t n_item
     }
 }
 
-// one warp per option: Re sum_j W_q(j) disc K e^{-i u_j x}
-__global__ void price_kernel(const Exp *ex, const Item *items, uint32_t n_items, const double2 *W,
-                             const double *strikes, double *price, double *grad) {
-    const uint32_t it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (it >= n_items) return;
-    const Exp E = ex[items[it].e];
-    const uint32_t i = items[it].first, lane = threadIdx.x & 31u;
-    const double K = strikes[E.o_off + i];
-    const double x = E.r * E.tau + log(E.S / K);
+// One warp per option: Re sum_j W_q(j) disc K e^{-i u_j x}.  A lane's terms
+// are 32 j apart, so its phase turns by e^{-i 64 du x} from one to the next:
+// one complex product instead of a sincos (4 FP64 instructions instead of
+// about 45), and a sincos every 16 terms, so that the products' roundings do
+// not add up beyond the sincos argument's own.  kGrad: the gradient too.
+constexpr uint32_t kTurns = 16;
+template <bool kGrad>
+__global__ void __launch_bounds__(128) price_kernel(const Exp *ex, const Item *items, const double2 *W,
+                                                    const Opt *opts, double *price, double *grad) {
+    const Exp &E = ex[items[blockIdx.x].e];
+    const uint32_t i = items[blockIdx.x].first + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+    if (i >= E.n_opt) return;   // warp-uniform
+    const Opt o = opts[E.o_off + i];
+    constexpr int kQ = kGrad ? 6 : 1;
     double acc[6] = {0, 0, 0, 0, 0, 0};
-    for (uint32_t j = lane; j < E.J; j += 32) {
+    const uint32_t span = 32u * (E.stiff ? 1u : kTurns);
+    for (uint32_t j0 = lane; j0 < E.J; j0 += span) {
         double s, c;
-        sincos((2.0 * j + 1.0) * E.du * x, &s, &c);     // e^{-i u x} = c - i s
+        sincos((2.0 * j0 + 1.0) * E.du * o.x, &s, &c);     // e^{-i u x} = c - i s
+        const uint32_t j1 = min(E.J, j0 + span);
+        for (uint32_t j = j0; j < j1; j += 32) {
 #pragma unroll
-        for (int q = 0; q < 6; ++q) {
-            const double2 w = W[E.w_off + (uint64_t)q * E.J + j];
-            acc[q] = fma(w.x, c, fma(w.y, s, acc[q]));
+            for (int q = 0; q < kQ; ++q) {
+                const double2 w = W[E.w_off + (uint64_t)q * E.J + j];
+                acc[q] = fma(w.x, c, fma(w.y, s, acc[q]));
+            }
+            const double c1 = fma(c, o.tc, -s * o.ts);
+            s = fma(c, o.ts, s * o.tc);
+            c = c1;
         }
     }
+    if constexpr (kGrad) {   // lanes 0-15 take on the first three sums, 16-31 the others
+        const bool up = lane >= 16u;
 #pragma unroll
-    for (int q = 0; q < 6; ++q)
-        for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
-    if (lane == 0) {
-        const double f = exp(-E.r * E.tau) * K;
-        price[E.o_off + i] = f * acc[0];
-        if (grad != nullptr)
+        for (int q = 0; q < 3; ++q) {
+            const double mine = up ? acc[q + 3] : acc[q], theirs = up ? acc[q] : acc[q + 3];
+            acc[q] = mine + __shfl_xor_sync(0xffffffffu, theirs, 16);
+        }
+    } else {
+        acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 16);
+    }
 #pragma unroll
-            for (int q = 0; q < 5; ++q) grad[(E.o_off + i) * 5 + q] = f * acc[q + 1];
+    for (int q = 0; q < (kGrad ? 3 : 1); ++q)
+        for (int d = 8; d > 0; d >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], d);
+    if ((lane & 15u) == 0u) {
+        const double f = o.f;
+        if (lane == 0u) price[E.o_off + i] = f * acc[0];
+        if constexpr (kGrad) {
+            double *g = grad + (E.o_off + i) * 5;
+            if (lane == 0u) { g[0] = f * acc[1]; g[1] = f * acc[2]; }
+            else { g[2] = f * acc[0]; g[3] = f * acc[1]; g[4] = f * acc[2]; }
+        }
     }
 }
 
@@ -456,8 +666,11 @@ hexo_status hexo_swift_price(hexo_ctx *ctx, const hexo_swift_request *reqs, uint
     std::vector<double> strikes;
     std::vector<const hexo_swift_chain *> chain_of;
     uint64_t tw = 0, h = 0, v = 0, w = 0, f = 0;
-    uint32_t max_log = 0;
+    uint32_t max_part = 0;
     bool any_grad = false;
+    std::vector<Item> it_set, it_h, it_o, it_fft, it_pay, it_den, it_stiff, it_pri;
+    TwiddleAt tw_at;                        // ~0: no table yet
+    std::fill(tw_at.off, tw_at.off + 17, ~0ull);
     for (uint32_t q = 0; q < n_reqs; ++q) {
         const hexo_swift_request &rq = reqs[q];
         const HP hp{rq.params.v0, rq.params.theta, rq.params.rho, rq.params.kappa, rq.params.sigma};
@@ -486,14 +699,28 @@ hexo_status hexo_swift_price(hexo_ctx *ctx, const hexo_swift_request *reqs, uint
                 return ctx_fail(ctx, HEXO_ERR_UNSUPPORTED, "swift: J must be a power of two up to 65536 with k2 - k1 < 4J");
             if (ch.method > HEXO_SWIFT_FFT) return ctx_fail(ctx, HEXO_ERR_INVALID, "swift chain: unknown method");
             Exp e{};
-            e.fft = ch.method == HEXO_SWIFT_FFT || (ch.method == HEXO_SWIFT_AUTO && sp.J >= kFftMinJ);
-            if (e.fft) {   // two buffers of N = 2J
-                while ((1u << e.logN) < 2u * sp.J) ++e.logN;
-                e.f_off = f;
-                f += 4ull * sp.J;
-                max_log = std::max(max_log, e.logN);
+            uint32_t logJ = 0;
+            while ((1u << logJ) < sp.J) ++logJ;
+            e.stiff = sp.upper > kStiff;
+            if (ch.method == HEXO_SWIFT_FFT ||
+                (ch.method == HEXO_SWIFT_AUTO && sp.J >= (e.stiff ? kFftMinStiffJ : kFftMinJ))) {
+                e.logN = logJ + 1u;
+                e.logR = e.logN < 6u ? 0u : (uint32_t)std::max(kLogParts, (int)e.logN - kLogMaxPart);
+                e.y_off = f;
+                f += 2ull * sp.J;
+                max_part = std::max(max_part, 1u << (e.logN - e.logR));
+            } else {
+                e.v_off = v;
+                v += (uint64_t)(sp.k2 - sp.k1 + 1);
             }
+            if (tw_at.off[logJ] == ~0ull) {
+                tw_at.off[logJ] = tw;
+                for (uint32_t n = 0; n < 4 * sp.J; n += 128) it_set.push_back({logJ, n});
+                tw += 4ull * sp.J;
+            }
+            e.tw_off = tw_at.off[logJ];
             e.p = hp;
+            e.q = ChfConst{1.0 / hp.sigma, 2.0 * hp.kappa * hp.vm / (hp.sigma * hp.sigma), hp.rho / hp.sigma};
             e.tau = ch.tau;
             e.r = rq.params.r;
             e.S = rq.S;
@@ -505,29 +732,28 @@ hexo_status hexo_swift_price(hexo_ctx *ctx, const hexo_swift_request *reqs, uint
             e.k2 = sp.k2;
             e.J = sp.J;
             e.n_opt = ch.n;
-            e.tw_off = tw; tw += 4ull * sp.J;
             e.h_off = h; h += sp.J;
-            e.v_off = v; v += (uint64_t)(sp.k2 - sp.k1 + 1);
             e.w_off = w; w += 6ull * sp.J;
             e.o_off = strikes.size();
             strikes.insert(strikes.end(), ch.strikes, ch.strikes + ch.n);
+            const uint32_t at = (uint32_t)ex.size();
+            for (uint32_t j = 0; j < sp.J; j += 128) it_h.push_back({at, j});
+            if (e.logN)
+                for (uint32_t r = 0; r < (1u << e.logR); ++r) it_fft.push_back({at, r});
+            else
+                for (uint32_t k = 0; k < (uint32_t)(sp.k2 - sp.k1 + 1); k += 32) it_pay.push_back({at, k});
+            for (uint32_t j = 0; j < sp.J; j += 64) (e.stiff ? it_stiff : it_den).push_back({at, j});
+            for (uint32_t i = 0; i < ch.n; i += 128) it_o.push_back({at, i});
+            for (uint32_t i = 0; i < ch.n; i += 4) it_pri.push_back({at, i});
             ex.push_back(e);
             chain_of.push_back(&ch);
             any_grad |= ch.grad_out != nullptr;
         }
     }
     if (ex.empty()) return HEXO_OK;
-    std::vector<Item> it_tab, it_pay, it_den, it_pri, it_fn, it_fb;
-    for (uint32_t e = 0; e < ex.size(); ++e) {
-        for (uint32_t n = 0; n < 4 * ex[e].J; n += 32) it_tab.push_back({e, n});
-        for (uint32_t k = 0; k < (uint32_t)(ex[e].k2 - ex[e].k1 + 1); k += 32) it_pay.push_back({e, k});
-        for (uint32_t j = 0; j < ex[e].J; j += 32) it_den.push_back({e, j});
-        for (uint32_t i = 0; i < ex[e].n_opt; ++i) it_pri.push_back({e, i});
-        if (ex[e].fft) {
-            for (uint32_t n = 0; n < 2 * ex[e].J; n += 32) it_fn.push_back({e, n});   // N elements
-            for (uint32_t j = 0; j < ex[e].J; j += 32) it_fb.push_back({e, j});       // N/2 butterflies
-        }
-    }
+    const uint32_t n_tw = (uint32_t)it_set.size(), n_h = (uint32_t)it_h.size();
+    it_set.insert(it_set.end(), it_h.begin(), it_h.end());
+    it_set.insert(it_set.end(), it_o.begin(), it_o.end());
     const size_t n_opt = strikes.size();
     std::lock_guard<std::mutex> lk(ctx->run_mu);
     cudaSetDevice(ctx->device);
@@ -536,14 +762,13 @@ hexo_status hexo_swift_price(hexo_ctx *ctx, const hexo_swift_request *reqs, uint
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t o = off; off = (off + bytes + 255) / 256 * 256; return o; };
     const size_t o_ex = take(ex.size() * sizeof(Exp));
-    const size_t o_i1 = take(it_tab.size() * sizeof(Item)), o_i2 = take(it_pay.size() * sizeof(Item));
-    const size_t o_i3 = take(it_den.size() * sizeof(Item)), o_i4 = take(it_pri.size() * sizeof(Item));
-    const size_t o_k = take(n_opt * sizeof(double));
+    const size_t o_is = take(it_set.size() * sizeof(Item)), o_if = take(it_fft.size() * sizeof(Item));
+    const size_t o_ip = take(it_pay.size() * sizeof(Item)), o_id = take(it_den.size() * sizeof(Item));
+    const size_t o_it = take(it_stiff.size() * sizeof(Item)), o_ir = take(it_pri.size() * sizeof(Item));
+    const size_t o_k = take(n_opt * sizeof(double)), o_o = take(n_opt * sizeof(Opt));
     const size_t o_tw = take(tw * sizeof(double2)), o_h = take(h * sizeof(double2));
-    const size_t o_v = take(v * sizeof(double)), o_w = take(w * sizeof(double2));
+    const size_t o_v = take(v * sizeof(double)), o_w = take(w * sizeof(double2)), o_y = take(f * sizeof(double2)), o_z = take(f * sizeof(double2));
     const size_t o_p = take(n_opt * sizeof(double)), o_g = take(any_grad ? n_opt * 5 * sizeof(double) : 0);
-    const size_t o_i5 = take(it_fn.size() * sizeof(Item)), o_i6 = take(it_fb.size() * sizeof(Item));
-    const size_t o_f = take(f * sizeof(double2));
     void *dmem = nullptr;   // the context's arena: no allocation once it is large enough
     cudaError_t err = ctx_scratch(ctx, off, &dmem);
     if (err != cudaSuccess) return cuda_fail(ctx, err, "cudaMalloc swift");
@@ -551,42 +776,40 @@ hexo_status hexo_swift_price(hexo_ctx *ctx, const hexo_swift_request *reqs, uint
     auto up = [&](size_t o, const void *src, size_t bytes) {
         return bytes ? cudaMemcpyAsync(d + o, src, bytes, cudaMemcpyHostToDevice, st) : cudaSuccess;
     };
+    auto up_items = [&](size_t o, const std::vector<Item> &it) { return up(o, it.data(), it.size() * sizeof(Item)); };
     if ((err = up(o_ex, ex.data(), ex.size() * sizeof(Exp))) != cudaSuccess ||
-        (err = up(o_i1, it_tab.data(), it_tab.size() * sizeof(Item))) != cudaSuccess ||
-        (err = up(o_i2, it_pay.data(), it_pay.size() * sizeof(Item))) != cudaSuccess ||
-        (err = up(o_i3, it_den.data(), it_den.size() * sizeof(Item))) != cudaSuccess ||
-        (err = up(o_i4, it_pri.data(), it_pri.size() * sizeof(Item))) != cudaSuccess ||
-        (err = up(o_i5, it_fn.data(), it_fn.size() * sizeof(Item))) != cudaSuccess ||
-        (err = up(o_i6, it_fb.data(), it_fb.size() * sizeof(Item))) != cudaSuccess ||
+        (err = up_items(o_is, it_set)) != cudaSuccess || (err = up_items(o_if, it_fft)) != cudaSuccess ||
+        (err = up_items(o_ip, it_pay)) != cudaSuccess || (err = up_items(o_id, it_den)) != cudaSuccess ||
+        (err = up_items(o_it, it_stiff)) != cudaSuccess || (err = up_items(o_ir, it_pri)) != cudaSuccess ||
         (err = up(o_k, strikes.data(), n_opt * sizeof(double))) != cudaSuccess)
         return cuda_fail(ctx, err, "upload swift");
     const Exp *dex = reinterpret_cast<const Exp *>(d + o_ex);
+    auto items = [&](size_t o) { return reinterpret_cast<const Item *>(d + o); };
     double2 *dtw = reinterpret_cast<double2 *>(d + o_tw), *dh = reinterpret_cast<double2 *>(d + o_h);
     double *dv = reinterpret_cast<double *>(d + o_v);
-    double2 *dw = reinterpret_cast<double2 *>(d + o_w);
+    double2 *dw = reinterpret_cast<double2 *>(d + o_w), *dy = reinterpret_cast<double2 *>(d + o_y),
+            *dz = reinterpret_cast<double2 *>(d + o_z);
     double *dp = reinterpret_cast<double *>(d + o_p), *dg = any_grad ? reinterpret_cast<double *>(d + o_g) : nullptr;
-    double2 *df = reinterpret_cast<double2 *>(d + o_f);
-    const uint32_t n1 = (uint32_t)it_tab.size(), n2 = (uint32_t)it_pay.size(), n3 = (uint32_t)it_den.size(),
-                   n4 = (uint32_t)it_pri.size(), n5 = (uint32_t)it_fn.size(), n6 = (uint32_t)it_fb.size();
-    const Item *ifn = reinterpret_cast<const Item *>(d + o_i5), *ifb = reinterpret_cast<const Item *>(d + o_i6);
-    auto fft_passes = [&]() {
-        for (uint32_t pass = 0; pass < max_log; ++pass)
-            fft_pass_kernel<<<(n6 + 3) / 4, 128, 0, st>>>(dex, ifb, n6, pass, df);
-    };
-    tables_kernel<<<(n1 + 3) / 4, 128, 0, st>>>(dex, reinterpret_cast<const Item *>(d + o_i1), n1, dtw, dh);
-    if (n5) {   // F = IDFT(h) of the FFT expiries
-        fft_load_h_kernel<<<(n5 + 3) / 4, 128, 0, st>>>(dex, ifn, n5, dh, df);
-        fft_passes();
+    Opt *dopt = reinterpret_cast<Opt *>(d + o_o);
+    setup_kernel<<<(unsigned)it_set.size(), 128, 0, st>>>(dex, items(o_is), n_tw, n_h, tw_at,
+                                                          reinterpret_cast<const double *>(d + o_k), dtw, dh, dopt);
+    if (!it_fft.empty()) {
+        const size_t smem = max_part * sizeof(double2);
+        if (smem > 48u << 10)
+            for (const void *fn : {(const void *)fft_terms_kernel, (const void *)fft_payoff_kernel})
+                if ((err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)(sizeof(double2) << kLogMaxPart))) != cudaSuccess)
+                    return cuda_fail(ctx, err, "swift shared memory");
+        fft_terms_kernel<<<(unsigned)it_fft.size(), 128, smem, st>>>(dex, items(o_if), dtw, dh, dy);
+        fft_payoff_kernel<<<(unsigned)it_fft.size(), 128, smem, st>>>(dex, items(o_if), dtw, dy, dz);
     }
-    payoff_kernel<<<(n2 + 3) / 4, 128, 0, st>>>(dex, reinterpret_cast<const Item *>(d + o_i2), n2, dtw, dh, dv, df);
-    if (n5) {   // G = IDFT(folded V w^k)
-        fft_load_g_kernel<<<(n5 + 3) / 4, 128, 0, st>>>(dex, ifn, n5, dtw, dv, df);
-        fft_passes();
-    }
-    density_kernel<<<(n3 + 3) / 4, 128, 0, st>>>(dex, reinterpret_cast<const Item *>(d + o_i3), n3, dtw, dv, dw,
-                                                 df);
-    price_kernel<<<(n4 + 3) / 4, 128, 0, st>>>(dex, reinterpret_cast<const Item *>(d + o_i4), n4, dw,
-                                               reinterpret_cast<const double *>(d + o_k), dp, dg);
+    if (!it_pay.empty()) payoff_kernel<<<(unsigned)it_pay.size(), 32, 0, st>>>(dex, items(o_ip), dtw, dh, dv);
+    if (!it_den.empty())
+        density_kernel<false><<<(unsigned)it_den.size(), 64, 0, st>>>(dex, items(o_id), dtw, dv, dw, dz);
+    if (!it_stiff.empty())
+        density_kernel<true><<<(unsigned)it_stiff.size(), 64, 0, st>>>(dex, items(o_it), dtw, dv, dw, dz);
+    if (any_grad) price_kernel<true><<<(unsigned)it_pri.size(), 128, 0, st>>>(dex, items(o_ir), dw, dopt, dp, dg);
+    else price_kernel<false><<<(unsigned)it_pri.size(), 128, 0, st>>>(dex, items(o_ir), dw, dopt, dp, dg);
     if ((err = cudaGetLastError()) != cudaSuccess) return cuda_fail(ctx, err, "swift kernels");
     std::vector<double> hp(n_opt), hg(any_grad ? n_opt * 5 : 0);
     if ((err = cudaMemcpyAsync(hp.data(), dp, n_opt * sizeof(double), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
