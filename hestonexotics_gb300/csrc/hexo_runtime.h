@@ -139,6 +139,24 @@ inline cudaError_t ctx_scratch(hexo_ctx *ctx, size_t bytes, void **p) {
     return cudaSuccess;
 }
 
+// The context's pinned host arena likewise; null when `bytes` is more than is
+// kept between calls or cannot be had (the caller then uses pageable memory).
+inline void *ctx_scratch_host(hexo_ctx *ctx, size_t bytes) {
+    if (bytes > kArenaKeepBytes) return nullptr;
+    if (ctx->arena_h == nullptr || ctx->arena_hcap < bytes) {
+        if (ctx->arena_h) cudaFreeHost(ctx->arena_h);
+        ctx->arena_h = nullptr;
+        ctx->arena_hcap = 0;
+        if (cudaMallocHost(&ctx->arena_h, bytes ? bytes : 1) != cudaSuccess) {
+            (void)cudaGetLastError();
+            ctx->arena_h = nullptr;
+            return nullptr;
+        }
+        ctx->arena_hcap = bytes;
+    }
+    return ctx->arena_h;
+}
+
 hexo_status ctx_fail(hexo_ctx *ctx, hexo_status s, const std::string &msg);
 hexo_status cuda_fail(hexo_ctx *ctx, cudaError_t e, const char *what);
 LaunchShape ctx_shape(hexo_ctx *ctx, const hexo_mc_cfg &cfg);

@@ -23,6 +23,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "hexo_mc.h"
@@ -230,10 +231,27 @@ static __device__ __noinline__ void chf_grad_far(const HP &p, double tau, double
 
 // ------------------------------------------------ dynamic wavelet parameters
 
+// Every operation is odd or even in the sign of the frequency, so phi(-u) is
+// the conjugate of phi(u) bit for bit and |phi(u) + phi(-u)| = 2 |Re phi(u)|;
+// phi alone needs neither B nor the hyperbolic functions twice.
 double int_error(const HP &p, double tau, unsigned m) {   // HDistribution.cpp:8-11
     const double e = std::exp2((double)m);
-    const cplx u1 = C(e * M_PI), u2 = C(-e * M_PI);
-    return cabs_(chf(p, tau, u1, aux(p, u1, tau)) + chf(p, tau, u2, aux(p, u2, tau))) / (4.0 * e * M_PI * M_PI * tau);
+    const cplx u = C(e * M_PI), I = C(0.0, 1.0);
+    Aux a;
+    a.xi = p.kappa + p.sigma * p.rho * (I * u);
+    const cplx f = u * u - I * u;
+    a.d = csqrt_(a.xi * a.xi + p.sigma * p.sigma * f);
+    const cplx dt = a.d * (tau * 0.5);
+    const double sh = sinh(dt.re), ch = cosh(dt.re), sn = sin(dt.im), cs = cos(dt.im);
+    a.sh = C(sh * cs, ch * sn);
+    a.ch = C(ch * cs, sh * sn);
+    a.A1 = f * a.sh;
+    a.A2 = a.d / p.v0 * a.ch + a.xi / p.v0 * a.sh;
+    a.A = a.A1 / a.A2;
+    a.D = clog_((2.0 * a.d) / (a.d + a.xi + (a.d - a.xi) * cexp_(-(a.d * tau)))) + (p.kappa - a.d) * (tau * 0.5);
+    const cplx c = chf(p, tau, u, a);
+    const double s = std::isfinite(c.im) ? std::fabs(2.0 * c.re) : std::isinf(c.re) ? HUGE_VAL : std::nan("");
+    return s / (4.0 * e * M_PI * M_PI * tau);
 }
 
 // Cumulants (HDistribution.cpp:86-113).  The reference binds its parameter
@@ -640,6 +658,46 @@ hexo_status params_dynamic(const HP &p, double tau, double r, double S, double K
     return HEXO_OK;
 }
 
+// A chain to price, and its wavelet parameters.
+struct Pending {
+    const hexo_swift_chain *ch;
+    HP p;
+    double r, S, kmin, kmax;
+    hexo_swift_params sp;
+    hexo_status status;
+};
+
+// Chooses the wavelet parameters of chains [lo, hi) that do not bring their own.
+void choose_params(Pending *q, size_t lo, size_t hi) {
+    for (size_t i = lo; i < hi; ++i) {
+        Pending &c = q[i];
+        c.status = HEXO_OK;
+        if (c.ch->params) c.sp = *c.ch->params;
+        else
+            c.status = params_dynamic(c.p, c.ch->tau, c.r, c.S, c.kmin, c.kmax,
+                                      c.ch->trunc_precision > 0.0 ? c.ch->trunc_precision : 1e-7, c.sp);
+    }
+}
+
+// The same over several threads, from 128 chains a thread on: the truncation
+// loop takes 1 to 2 us a chain, and starting a thread about 20 us (a surface
+// of 2,048 chains: 2.4 ms on one thread, as long as its kernels).
+void choose_params_all(std::vector<Pending> &q) {
+    const size_t n = q.size(), most = std::min<size_t>({8u, std::max(1u, std::thread::hardware_concurrency()), n / 128u + 1u});
+    std::vector<std::thread> ts;
+    size_t lo = 0;
+    try {
+        for (size_t t = 1; t < most; ++t) {
+            const size_t hi = n * t / most;
+            ts.emplace_back(choose_params, q.data(), lo, hi);
+            lo = hi;
+        }
+    } catch (...) {   // no thread to be had: the rest runs here
+    }
+    choose_params(q.data(), lo, n);
+    for (std::thread &t : ts) t.join();
+}
+
 bool valid_params(const hexo_swift_params &sp) {
     const uint32_t J = sp.J;
     return J >= 1 && J <= kMaxJ && (J & (J - 1)) == 0 && sp.k1 <= sp.k2 &&
@@ -671,85 +729,94 @@ hexo_status hexo_swift_price(hexo_ctx *ctx, const hexo_swift_request *reqs, uint
     std::vector<Item> it_set, it_h, it_o, it_fft, it_pay, it_den, it_stiff, it_pri;
     TwiddleAt tw_at;                        // ~0: no table yet
     std::fill(tw_at.off, tw_at.off + 17, ~0ull);
-    for (uint32_t q = 0; q < n_reqs; ++q) {
+    // the chains up to the first that is refused, whose error is returned after theirs
+    std::vector<Pending> todo;
+    std::string refused;
+    for (uint32_t q = 0; q < n_reqs && refused.empty(); ++q) {
         const hexo_swift_request &rq = reqs[q];
         const HP hp{rq.params.v0, rq.params.theta, rq.params.rho, rq.params.kappa, rq.params.sigma};
         if (!(hp.v0 > 0.0) || !(hp.sigma > 0.0) || !(hp.kappa > 0.0) || !(rq.S > 0.0) ||
-            !std::isfinite(rq.params.r) || (rq.n_chains > 0 && !rq.chains))
-            return ctx_fail(ctx, HEXO_ERR_INVALID, "swift request " + std::to_string(q) + ": bad parameters");
-        for (uint32_t c = 0; c < rq.n_chains; ++c) {
+            !std::isfinite(rq.params.r) || (rq.n_chains > 0 && !rq.chains)) {
+            refused = "swift request " + std::to_string(q) + ": bad parameters";
+            break;
+        }
+        for (uint32_t c = 0; c < rq.n_chains && refused.empty(); ++c) {
             const hexo_swift_chain &ch = rq.chains[c];
             if (ch.n == 0) continue;
-            if (!ch.strikes || !ch.price_out || !(ch.tau > 0.0))
-                return ctx_fail(ctx, HEXO_ERR_INVALID, "swift chain: missing strikes/outputs or tau <= 0");
-            double kmin = ch.strikes[0], kmax = ch.strikes[0];
+            if (!ch.strikes || !ch.price_out || !(ch.tau > 0.0)) {
+                refused = "swift chain: missing strikes/outputs or tau <= 0";
+                break;
+            }
+            Pending p{&ch, hp, rq.params.r, rq.S, ch.strikes[0], ch.strikes[0], {}, HEXO_OK};
             for (uint32_t i = 0; i < ch.n; ++i) {
-                if (!(ch.strikes[i] > 0.0)) return ctx_fail(ctx, HEXO_ERR_INVALID, "swift chain: strike <= 0");
-                kmin = std::min(kmin, ch.strikes[i]);
-                kmax = std::max(kmax, ch.strikes[i]);
+                if (!(ch.strikes[i] > 0.0)) refused = "swift chain: strike <= 0";
+                p.kmin = std::min(p.kmin, ch.strikes[i]);
+                p.kmax = std::max(p.kmax, ch.strikes[i]);
             }
-            hexo_swift_params sp;
-            if (ch.params) sp = *ch.params;
-            else {
-                const double prec = ch.trunc_precision > 0.0 ? ch.trunc_precision : 1e-7;
-                const hexo_status s = params_dynamic(hp, ch.tau, rq.params.r, rq.S, kmin, kmax, prec, sp);
-                if (s != HEXO_OK) return ctx_fail(ctx, s, "swift: the truncation loop did not converge");
-            }
-            if (!valid_params(sp))
-                return ctx_fail(ctx, HEXO_ERR_UNSUPPORTED, "swift: J must be a power of two up to 65536 with k2 - k1 < 4J");
-            if (ch.method > HEXO_SWIFT_FFT) return ctx_fail(ctx, HEXO_ERR_INVALID, "swift chain: unknown method");
-            Exp e{};
-            uint32_t logJ = 0;
-            while ((1u << logJ) < sp.J) ++logJ;
-            e.stiff = sp.upper > kStiff;
-            if (ch.method == HEXO_SWIFT_FFT ||
-                (ch.method == HEXO_SWIFT_AUTO && sp.J >= (e.stiff ? kFftMinStiffJ : kFftMinJ))) {
-                e.logN = logJ + 1u;
-                e.logR = e.logN < 6u ? 0u : (uint32_t)std::max(kLogParts, (int)e.logN - kLogMaxPart);
-                e.y_off = f;
-                f += 2ull * sp.J;
-                max_part = std::max(max_part, 1u << (e.logN - e.logR));
-            } else {
-                e.v_off = v;
-                v += (uint64_t)(sp.k2 - sp.k1 + 1);
-            }
-            if (tw_at.off[logJ] == ~0ull) {
-                tw_at.off[logJ] = tw;
-                for (uint32_t n = 0; n < 4 * sp.J; n += 128) it_set.push_back({logJ, n});
-                tw += 4ull * sp.J;
-            }
-            e.tw_off = tw_at.off[logJ];
-            e.p = hp;
-            e.q = ChfConst{1.0 / hp.sigma, 2.0 * hp.kappa * hp.vm / (hp.sigma * hp.sigma), hp.rho / hp.sigma};
-            e.tau = ch.tau;
-            e.r = rq.params.r;
-            e.S = rq.S;
-            e.sqrt2m = sp.sqrt_exp2_m;
-            e.lower = sp.lower;
-            e.upper = sp.upper;
-            e.du = M_PI * (double)sp.exp2_m / (2.0 * sp.J);
-            e.k1 = sp.k1;
-            e.k2 = sp.k2;
-            e.J = sp.J;
-            e.n_opt = ch.n;
-            e.h_off = h; h += sp.J;
-            e.w_off = w; w += 6ull * sp.J;
-            e.o_off = strikes.size();
-            strikes.insert(strikes.end(), ch.strikes, ch.strikes + ch.n);
-            const uint32_t at = (uint32_t)ex.size();
-            for (uint32_t j = 0; j < sp.J; j += 128) it_h.push_back({at, j});
-            if (e.logN)
-                for (uint32_t r = 0; r < (1u << e.logR); ++r) it_fft.push_back({at, r});
-            else
-                for (uint32_t k = 0; k < (uint32_t)(sp.k2 - sp.k1 + 1); k += 32) it_pay.push_back({at, k});
-            for (uint32_t j = 0; j < sp.J; j += 64) (e.stiff ? it_stiff : it_den).push_back({at, j});
-            for (uint32_t i = 0; i < ch.n; i += 128) it_o.push_back({at, i});
-            for (uint32_t i = 0; i < ch.n; i += 4) it_pri.push_back({at, i});
-            ex.push_back(e);
-            chain_of.push_back(&ch);
-            any_grad |= ch.grad_out != nullptr;
+            if (refused.empty()) todo.push_back(p);
         }
     }
+    choose_params_all(todo);
+    for (const Pending &pd : todo) {
+        const hexo_swift_chain &ch = *pd.ch;
+        const HP &hp = pd.p;
+        const hexo_swift_params &sp = pd.sp;
+        if (pd.status != HEXO_OK) return ctx_fail(ctx, pd.status, "swift: the truncation loop did not converge");
+        if (!valid_params(sp))
+            return ctx_fail(ctx, HEXO_ERR_UNSUPPORTED, "swift: J must be a power of two up to 65536 with k2 - k1 < 4J");
+        if (ch.method > HEXO_SWIFT_FFT) return ctx_fail(ctx, HEXO_ERR_INVALID, "swift chain: unknown method");
+        Exp e{};
+        uint32_t logJ = 0;
+        while ((1u << logJ) < sp.J) ++logJ;
+        e.stiff = sp.upper > kStiff;
+        if (ch.method == HEXO_SWIFT_FFT ||
+            (ch.method == HEXO_SWIFT_AUTO && sp.J >= (e.stiff ? kFftMinStiffJ : kFftMinJ))) {
+            e.logN = logJ + 1u;
+            e.logR = e.logN < 6u ? 0u : (uint32_t)std::max(kLogParts, (int)e.logN - kLogMaxPart);
+            e.y_off = f;
+            f += 2ull * sp.J;
+            max_part = std::max(max_part, 1u << (e.logN - e.logR));
+        } else {
+            e.v_off = v;
+            v += (uint64_t)(sp.k2 - sp.k1 + 1);
+        }
+        if (tw_at.off[logJ] == ~0ull) {
+            tw_at.off[logJ] = tw;
+            for (uint32_t n = 0; n < 4 * sp.J; n += 128) it_set.push_back({logJ, n});
+            tw += 4ull * sp.J;
+        }
+        e.tw_off = tw_at.off[logJ];
+        e.p = hp;
+        e.q = ChfConst{1.0 / hp.sigma, 2.0 * hp.kappa * hp.vm / (hp.sigma * hp.sigma), hp.rho / hp.sigma};
+        e.tau = ch.tau;
+        e.r = pd.r;
+        e.S = pd.S;
+        e.sqrt2m = sp.sqrt_exp2_m;
+        e.lower = sp.lower;
+        e.upper = sp.upper;
+        e.du = M_PI * (double)sp.exp2_m / (2.0 * sp.J);
+        e.k1 = sp.k1;
+        e.k2 = sp.k2;
+        e.J = sp.J;
+        e.n_opt = ch.n;
+        e.h_off = h; h += sp.J;
+        e.w_off = w; w += 6ull * sp.J;
+        e.o_off = strikes.size();
+        strikes.insert(strikes.end(), ch.strikes, ch.strikes + ch.n);
+        const uint32_t at = (uint32_t)ex.size();
+        for (uint32_t j = 0; j < sp.J; j += 128) it_h.push_back({at, j});
+        if (e.logN)
+            for (uint32_t r = 0; r < (1u << e.logR); ++r) it_fft.push_back({at, r});
+        else
+            for (uint32_t k = 0; k < (uint32_t)(sp.k2 - sp.k1 + 1); k += 32) it_pay.push_back({at, k});
+        for (uint32_t j = 0; j < sp.J; j += 64) (e.stiff ? it_stiff : it_den).push_back({at, j});
+        for (uint32_t i = 0; i < ch.n; i += 128) it_o.push_back({at, i});
+        for (uint32_t i = 0; i < ch.n; i += 4) it_pri.push_back({at, i});
+        ex.push_back(e);
+        chain_of.push_back(&ch);
+        any_grad |= ch.grad_out != nullptr;
+    }
+    if (!refused.empty()) return ctx_fail(ctx, HEXO_ERR_INVALID, refused);
     if (ex.empty()) return HEXO_OK;
     const uint32_t n_tw = (uint32_t)it_set.size(), n_h = (uint32_t)it_h.size();
     it_set.insert(it_set.end(), it_h.begin(), it_h.end());
@@ -758,30 +825,41 @@ hexo_status hexo_swift_price(hexo_ctx *ctx, const hexo_swift_request *reqs, uint
     std::lock_guard<std::mutex> lk(ctx->run_mu);
     cudaSetDevice(ctx->device);
     cudaStream_t st = ctx->stream;
-    // one allocation: descriptors, items, tables, outputs
+    // one allocation: what is uploaded (one copy), work buffers, outputs (one copy back)
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t o = off; off = (off + bytes + 255) / 256 * 256; return o; };
     const size_t o_ex = take(ex.size() * sizeof(Exp));
     const size_t o_is = take(it_set.size() * sizeof(Item)), o_if = take(it_fft.size() * sizeof(Item));
     const size_t o_ip = take(it_pay.size() * sizeof(Item)), o_id = take(it_den.size() * sizeof(Item));
     const size_t o_it = take(it_stiff.size() * sizeof(Item)), o_ir = take(it_pri.size() * sizeof(Item));
-    const size_t o_k = take(n_opt * sizeof(double)), o_o = take(n_opt * sizeof(Opt));
+    const size_t o_k = take(n_opt * sizeof(double)), up_bytes = off;
+    const size_t o_o = take(n_opt * sizeof(Opt));
     const size_t o_tw = take(tw * sizeof(double2)), o_h = take(h * sizeof(double2));
-    const size_t o_v = take(v * sizeof(double)), o_w = take(w * sizeof(double2)), o_y = take(f * sizeof(double2)), o_z = take(f * sizeof(double2));
+    const size_t o_v = take(v * sizeof(double)), o_w = take(w * sizeof(double2));
+    const size_t o_y = take(f * sizeof(double2)), o_z = take(f * sizeof(double2));
     const size_t o_p = take(n_opt * sizeof(double)), o_g = take(any_grad ? n_opt * 5 * sizeof(double) : 0);
+    const size_t down_bytes = off - o_p;
     void *dmem = nullptr;   // the context's arena: no allocation once it is large enough
     cudaError_t err = ctx_scratch(ctx, off, &dmem);
     if (err != cudaSuccess) return cuda_fail(ctx, err, "cudaMalloc swift");
     char *d = static_cast<char *>(dmem);
-    auto up = [&](size_t o, const void *src, size_t bytes) {
-        return bytes ? cudaMemcpyAsync(d + o, src, bytes, cudaMemcpyHostToDevice, st) : cudaSuccess;
-    };
-    auto up_items = [&](size_t o, const std::vector<Item> &it) { return up(o, it.data(), it.size() * sizeof(Item)); };
-    if ((err = up(o_ex, ex.data(), ex.size() * sizeof(Exp))) != cudaSuccess ||
-        (err = up_items(o_is, it_set)) != cudaSuccess || (err = up_items(o_if, it_fft)) != cudaSuccess ||
-        (err = up_items(o_ip, it_pay)) != cudaSuccess || (err = up_items(o_id, it_den)) != cudaSuccess ||
-        (err = up_items(o_it, it_stiff)) != cudaSuccess || (err = up_items(o_ir, it_pri)) != cudaSuccess ||
-        (err = up(o_k, strikes.data(), n_opt * sizeof(double))) != cudaSuccess)
+    std::vector<char> pageable;
+    char *host = static_cast<char *>(ctx_scratch_host(ctx, std::max(up_bytes, down_bytes)));
+    if (host == nullptr) {
+        pageable.resize(std::max(up_bytes, down_bytes));
+        host = pageable.data();
+    }
+    auto put = [&](size_t o, const void *src, size_t bytes) { if (bytes) std::memcpy(host + o, src, bytes); };
+    auto put_items = [&](size_t o, const std::vector<Item> &it) { put(o, it.data(), it.size() * sizeof(Item)); };
+    put(o_ex, ex.data(), ex.size() * sizeof(Exp));
+    put_items(o_is, it_set);
+    put_items(o_if, it_fft);
+    put_items(o_ip, it_pay);
+    put_items(o_id, it_den);
+    put_items(o_it, it_stiff);
+    put_items(o_ir, it_pri);
+    put(o_k, strikes.data(), n_opt * sizeof(double));
+    if ((err = cudaMemcpyAsync(d, host, up_bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess)
         return cuda_fail(ctx, err, "upload swift");
     const Exp *dex = reinterpret_cast<const Exp *>(d + o_ex);
     auto items = [&](size_t o) { return reinterpret_cast<const Item *>(d + o); };
@@ -811,16 +889,14 @@ hexo_status hexo_swift_price(hexo_ctx *ctx, const hexo_swift_request *reqs, uint
     if (any_grad) price_kernel<true><<<(unsigned)it_pri.size(), 128, 0, st>>>(dex, items(o_ir), dw, dopt, dp, dg);
     else price_kernel<false><<<(unsigned)it_pri.size(), 128, 0, st>>>(dex, items(o_ir), dw, dopt, dp, dg);
     if ((err = cudaGetLastError()) != cudaSuccess) return cuda_fail(ctx, err, "swift kernels");
-    std::vector<double> hp(n_opt), hg(any_grad ? n_opt * 5 : 0);
-    if ((err = cudaMemcpyAsync(hp.data(), dp, n_opt * sizeof(double), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
-        (any_grad && (err = cudaMemcpyAsync(hg.data(), dg, n_opt * 5 * sizeof(double), cudaMemcpyDeviceToHost, st)) !=
-                         cudaSuccess) ||
+    if ((err = cudaMemcpyAsync(host, dp, down_bytes, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
         (err = cudaStreamSynchronize(st)) != cudaSuccess)
         return cuda_fail(ctx, err, "swift results");
+    const double *hp = reinterpret_cast<const double *>(host), *hg = reinterpret_cast<const double *>(host + (o_g - o_p));
     for (size_t e = 0; e < ex.size(); ++e) {
         const hexo_swift_chain &ch = *chain_of[e];
-        std::memcpy(ch.price_out, hp.data() + ex[e].o_off, ch.n * sizeof(double));
-        if (ch.grad_out) std::memcpy(ch.grad_out, hg.data() + ex[e].o_off * 5, ch.n * 5 * sizeof(double));
+        std::memcpy(ch.price_out, hp + ex[e].o_off, ch.n * sizeof(double));
+        if (ch.grad_out) std::memcpy(ch.grad_out, hg + ex[e].o_off * 5, ch.n * 5 * sizeof(double));
     }
     return HEXO_OK;
 }
