@@ -129,8 +129,8 @@ SegDesc na_segment(const hexo_params &p, double dt) {
     s.f_c = (float)(0.5 * dt * (p.kappa * p.rho / p.sigma - 0.5));
     ds_split(s.disc, s.ds_disc);
     ds_split(p.theta * (1.0 - s.disc), s.ds_m0);
-    ds_split(s.cA, s.ds_cA);
-    ds_split(s.cB, s.ds_cB);
+    ds_split(0.5 * s.cA, s.ds_hA);
+    ds_split(0.5 * s.cB, s.ds_hB);
     return s;
 }
 

@@ -76,8 +76,59 @@ __device__ __forceinline__ bool qe_step(PathVars<false> &pv, const SegDesc &sg, 
     return quad;
 }
 
+// The FP32 form's branches, m and hs = s^2/2 in double-single, m^2 = p + e.
+// As in the FP64 form (hexo_f64.cuh) the quadratic branch is (sqrt(c) + z
+// sqrt(a))^2 with c = sqrt(m^2 - hs) and a = hs / (m + c): 55 instructions and
+// four MUFU, against 95 for a (b + z)^2 in the reference's order, and no less
+// exact (relative error 2^-45 rms, 2^-44.5 before, the same largest).  The
+// roots and the quotient between stay unnormalised: their low parts are below
+// 2^-22 of the high ones, and what that adds to the next correction is below
+// the rounding that remains.
+__device__ __forceinline__ ds::F2 variance_quadratic(ds::F2 m, ds::F2 hs, float p, float e, float z) {
+    const float D = __fsub_rn(p, hs.h);                                  // m^2 - hs > m^2 / 4
+    const float Dl = __fadd_rn(__fsub_rn(__fsub_rn(p, D), hs.h), __fsub_rn(e, hs.l));
+    const float r1 = ds::rsqrt_approx(D), c = __fmul_rn(D, r1);
+    const float cl = __fmul_rn(__fadd_rn(__fmaf_rn(-c, c, D), Dl), __fmul_rn(0.5f, r1));
+    const float r2 = ds::rsqrt_approx(c), b = __fmul_rn(c, r2);          // sqrt(c)
+    const float bl = __fmul_rn(__fadd_rn(__fmaf_rn(-b, b, c), cl), __fmul_rn(0.5f, r2));
+    const float g = __fadd_rn(m.h, c);                                   // m + c, m >= c
+    const float gl = __fadd_rn(__fsub_rn(c, __fsub_rn(g, m.h)), __fadd_rn(m.l, cl));
+    const float rg = ds::rcp_approx(g), a = __fmul_rn(hs.h, rg);
+    const float al = __fmul_rn(__fmaf_rn(-a, gl, __fadd_rn(__fmaf_rn(-a, g, hs.h), hs.l)), rg);
+    const float r3 = ds::rsqrt_approx(a), s = __fmul_rn(a, r3);          // sqrt(a)
+    const float sl = __fmul_rn(__fadd_rn(__fmaf_rn(-s, s, a), al), __fmul_rn(0.5f, r3));
+    const float q = __fmul_rn(z, s), ql = __fmaf_rn(z, sl, __fmaf_rn(z, s, -q));
+    const ds::F2 w = ds::two_sum(b, q);
+    return ds::sqr(ds::fast_two_sum(w.h, __fadd_rn(w.l, __fadd_rn(bl, ql))));
+}
+
+// -m Y log(Y (1 - U)), Y = (hs + m^2/2) / m^2, 1 - U = (2^64 - w) 2^-64 from
+// the whole word, or 0 where p >= U: that is where Y (1 - U) >= 1, since Y =
+// 1 / (1 - p).  The value is continuous there, so it does not matter that the
+// FP64 form may round a tie the other way.  In double-single like the
+// quadratic branch: a float-size error here would move later branch
+// decisions.
+__device__ __forceinline__ ds::F2 variance_exponential(ds::F2 m, ds::F2 hs, float p, float e, uint64_t uw,
+                                                       const ds::LogTab *ltab) {
+    const float W = __fmaf_rn(0.5f, p, hs.h);                            // hs >= 0.75 m^2
+    const float Wl = __fadd_rn(__fmaf_rn(0.5f, p, __fsub_rn(hs.h, W)), __fmaf_rn(0.5f, e, hs.l));
+    const float rp = ds::rcp_approx(p), y = __fmul_rn(W, rp);
+    const float yl = __fmul_rn(__fmaf_rn(-y, e, __fadd_rn(__fmaf_rn(-y, p, W), Wl)), rp);
+    const ds::F2 om = ds::from_u64_2m64(0ull - uw);
+    const float x = __fmul_rn(y, om.h);
+    const ds::F2 X = ds::fast_two_sum(x, __fmaf_rn(yl, om.h, __fmaf_rn(y, om.l, __fmaf_rn(y, om.h, -x))));
+    ds::F2 vn{0.0f, 0.0f};
+    if (uw != 0ull && (X.h < 1.0f || (X.h == 1.0f && X.l < 0.0f))) {     // U = 0 is never above p
+        const float mY = __fmul_rn(m.h, y);
+        const ds::F2 M{mY, __fmaf_rn(m.l, y, __fmaf_rn(m.h, yl, __fmaf_rn(m.h, y, -mY)))};
+        const ds::F2 v1 = ds::mul(M, ds::neg(ds::log(X, ltab)));
+        if (v1.h > 0.0f) vn = v1;
+    }
+    return vn;
+}
+
 // One QE step, FP32 form: the same scheme and draws; the variance in
-// double-single (m = v disc + m0 and s^2 = v cA + cB, algebraically the
+// double-single (m = v disc + m0 and s^2/2 = v cA/2 + cB/2, algebraically the
 // reference's tpp:59-60), everything else in float; returns whether it took
 // the quadratic branch.
 __device__ __forceinline__ bool qe_step(PathVars<true> &pv, const SegDesc &sg, dev::Shishua &g, dev::RngLane &c,
@@ -86,53 +137,22 @@ __device__ __forceinline__ bool qe_step(PathVars<true> &pv, const SegDesc &sg, d
     dev::DrawPlan dp = dev::draw_prefetch(c, r);
     const ds::F2 v = pv.vd;
     const ds::F2 m = ds::fma(v, ds::F2{sg.ds_disc[0], sg.ds_disc[1]}, ds::F2{sg.ds_m0[0], sg.ds_m0[1]});
-    const ds::F2 sp2 = ds::fma(v, ds::F2{sg.ds_cA[0], sg.ds_cA[1]}, ds::F2{sg.ds_cB[0], sg.ds_cB[1]});
-    const ds::F2 mm = ds::sqr(m);
-    // Psi < PSI_C; the float comparison decides unless it is within 2^-20 of the threshold
-    const float t15 = __fmul_rn(1.5f, mm.h);
-    const bool quad = fabsf(__fsub_rn(sp2.h, t15)) > __fmul_rn(0x1p-20f, sp2.h) ? sp2.h < t15
-                                                                                 : ds::less(sp2, ds::mul_f(mm, 1.5f));
+    const ds::F2 hs = ds::fma(v, ds::F2{sg.ds_hA[0], sg.ds_hA[1]}, ds::F2{sg.ds_hB[0], sg.ds_hB[1]});   // s^2 / 2
+    // m^2 as p + e, not normalised
+    const float p = __fmul_rn(m.h, m.h);
+    const float e = __fmaf_rn(__fadd_rn(m.h, m.h), m.l, __fmaf_rn(m.h, m.h, -p));
+    // Psi < PSI_C, s^2/2 < 0.75 m^2; the float comparison decides unless it is within 2^-20 of the threshold
+    const float t75 = __fmul_rn(0.75f, p);
+    const bool quad = fabsf(__fsub_rn(hs.h, t75)) > __fmul_rn(0x1p-20f, hs.h)
+                          ? hs.h < t75
+                          : ds::less(hs, ds::mul_f(ds::fast_two_sum(p, e), 0.75f));
     if (dev::draw_prepare<true>(g, c, r, ws, quad)) dp = dev::draw_prefetch(c, r);
     float z1 = 0.0f, z2;
     uint64_t uw = 0;
     dev::draw_commit(g, c, r, dp, quad, z1, uw, z2);
     ds::F2 vn;
-    if (quad) {
-        const ds::F2 inv = ds::div(ds::F2{__fmul_rn(2.0f, mm.h), __fmul_rn(2.0f, mm.l)}, sp2);   // 2/Psi
-        // inv > 4/3, sqrt(inv (inv - 1)) > inv - 1 and bp2 >= 1 order the additions
-        const ds::F2 im1 = ds::add_f_ordered(inv, -1.0f);
-        const ds::F2 bp2 = ds::add_ordered(ds::sqrt(ds::mul(inv, im1)), im1);
-        const ds::F2 b = ds::sqrt(bp2);
-        const ds::F2 a = ds::div(m, ds::add_f_ordered(bp2, 1.0f));
-        const ds::F2 zb = ds::add_f(b, z1);
-        vn = ds::mul(ds::mul(a, zb), zb);
-    } else {
-        const float Psi = __fdividef(sp2.h, mm.h);
-        const float pp1 = __fadd_rn(Psi, 1.0f);
-        const float p = __fdividef(__fsub_rn(Psi, 1.0f), pp1);
-        // U = w 2^-64 to float accuracy from the two 32-bit halves
-        const uint32_t whi = (uint32_t)(uw >> 32), wlo = (uint32_t)uw;
-        const float U = __fmaf_rn(__uint2float_rn(wlo), 0x1p-64f, __fmul_rn(__uint2float_rn(whi), 0x1p-32f));
-        // p < U sends the variance to 0 or not: decided in float when the two
-        // are further apart than float error (2^-19 relative), else exactly as
-        // the FP64 form decides it (rare: a few 1e-5 of these steps), so that
-        // the path does not take the other branch than in FP64
-        bool take = p < U;
-        if (fabsf(__fsub_rn(p, U)) <= __fmul_rn(0x1p-17f, __fadd_rn(p, U))) {
-            const double Pd = __ddiv_rn(__dadd_rn((double)sp2.h, (double)sp2.l), __dadd_rn((double)mm.h, (double)mm.l));
-            take = __ddiv_rn(__dsub_rn(Pd, 1.0), __dadd_rn(Pd, 1.0)) < dev::uniform_f64(uw);
-        }
-        // v = log((1-p)/(1-U)) / beta, in double-single like the quadratic
-        // branch (a float-size error here would move later branch decisions).
-        // With Y = (s^2 + m^2) / (2 m^2) = 1/(1-p) = 1/(beta m):
-        // v = -m Y log(Y (1 - U)), 1 - U = (2^64 - w) 2^-64 from the whole word
-        vn = ds::F2{0.0f, 0.0f};
-        if (take) {
-            const ds::F2 Y = ds::div(ds::add(sp2, mm), ds::F2{__fmul_rn(2.0f, mm.h), __fmul_rn(2.0f, mm.l)});
-            const ds::F2 v1 = ds::mul(ds::mul(m, Y), ds::neg(ds::log(ds::mul(Y, ds::from_u64_2m64(0ull - uw)), ltab)));
-            if (v1.h > 0.0f) vn = v1;
-        }
-    }
+    if (quad) vn = variance_quadratic(m, hs, p, e, z1);
+    else vn = variance_exponential(m, hs, p, e, uw, ltab);
     pv.vd = vn;
     pv.v = vn.h;
     // K1 v + K2 vn = c (v + vn) + (rho/sigma)(vn - v): the second part

@@ -60,8 +60,9 @@ struct SegDesc {
     float f_disc, f_cA, f_cB, f_K0, f_K1, f_K2, f_K3, f_K4, f_hdt, f_hdt_after;
     float f_c;      // 0.5 dt (kappa rho / sigma - 0.5): K1 = c - rho/sigma, K2 = c + rho/sigma
     float f_pad0;
-    // double-single (hi, lo) copies for the FP32 form's variance: m = v disc + m0, s^2 = v cA + cB
-    float ds_disc[2], ds_m0[2], ds_cA[2], ds_cB[2];
+    // double-single (hi, lo) copies for the FP32 form's variance: m = v disc + m0,
+    // s^2/2 = v hA + hB (hA = cA/2, hB = cB/2)
+    float ds_disc[2], ds_m0[2], ds_hA[2], ds_hB[2];
     uint32_t n_steps;   // steps in this segment, the last one prices
     uint32_t mat_begin; // maturities priced after the last step: [mat_begin, mat_end) (set-local)
     uint32_t mat_end;
