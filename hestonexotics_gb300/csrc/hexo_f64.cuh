@@ -252,6 +252,19 @@ __device__ __forceinline__ double root(double x) {
     return __longlong_as_double(__double_as_longlong(S) + (long long)k);
 }
 
+// z k within 0.51 ulp, z a float (0 gives a value below 2^-126 k) and k >= 0
+// normal, |z k| within the normal range: the 24- and 53-bit significands
+// multiplied in integers.
+__device__ __forceinline__ double mul_float(float z, double k) {
+    const uint32_t zb = __float_as_uint(z), kh = hi32(k), kl = lo32(k);
+    const uint32_t zm = zb << 8 | 0x80000000u;
+    uint64_t P = (uint64_t)zm * ((kh << 11 | kl >> 21) | 0x80000000u) + __umulhi(zm, kl << 11);
+    const uint32_t s = ~hi(P) >> 31;
+    P <<= s;
+    const uint32_t e = (kh >> 20) + (zb >> 23 & 0xffu) - 127u - s;   // the exponent field less one, which the leading bit adds
+    return __longlong_as_double((long long)((((uint64_t)(zb & 0x80000000u)) << 32) + ((uint64_t)e << 52) + ((P + 1024ull) >> 11)));
+}
+
 // 1 / x within 0.51 ulp, 2^-60 < x < 2^60, like root without an FP64 instruction.
 __device__ __forceinline__ double recip(double x) {
     const ds::F2 xs = split(x);
@@ -283,12 +296,18 @@ __device__ __forceinline__ bool in_range(double m, double s2) {
 }
 
 // Whether the step takes the quadratic branch, s2 < 1.5 m^2 (Psi < PSI_C,
-// HSimulation.tpp:61-63): in float unless the two are within 2^-20.
-__device__ __forceinline__ bool quadratic(double m, double s2) {
+// HSimulation.tpp:61-63): in float while in range and unless the two are
+// within 2^-20.  The exact comparison is a call so that it is not computed
+// ahead of the branch (three FP64 instructions in every step).
+static __device__ __noinline__ bool quadratic_exact(double m, double s2) {
+    return s2 < __dmul_rn(1.5, __dmul_rn(m, m));
+}
+__device__ __forceinline__ bool quadratic(double m, double s2, bool near) {
     const float mf = head(m), sf = head(s2);
     const float t = __fmul_rn(__fmul_rn(1.5f, mf), mf);
-    if (fabsf(__fsub_rn(sf, t)) > __fmul_rn(0x1p-20f, sf)) return sf < t;
-    return s2 < __dmul_rn(1.5, __dmul_rn(m, m));
+    bool quad = sf < t;
+    if (!near || !(fabsf(__fsub_rn(sf, t)) > __fmul_rn(0x1p-20f, sf))) quad = quadratic_exact(m, s2);
+    return quad;
 }
 
 // The quadratic branch a (b + z)^2 (HSimulation.tpp:64-68).  Its a and b

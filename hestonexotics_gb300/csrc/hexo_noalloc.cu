@@ -120,12 +120,13 @@ SegDesc na_segment(const hexo_params &p, double dt) {
     s.K0 = -p.rho * p.kappa * p.theta / p.sigma * dt + (p.r - p.q) * dt;
     s.K1 = 0.5 * dt * (p.kappa * p.rho / p.sigma - 0.5) - p.rho / p.sigma;
     s.K2 = 0.5 * dt * (p.kappa * p.rho / p.sigma - 0.5) + p.rho / p.sigma;
-    s.K3 = 0.5 * dt * (1.0 - p.rho * p.rho);
+    const double K3 = 0.5 * dt * (1.0 - p.rho * p.rho);
+    s.rK3 = std::max(std::sqrt(K3), 0x1p-200);
     s.m0 = p.theta * (1.0 - s.disc);
     s.hdt = dt * 0.5;
     s.f_disc = (float)s.disc; s.f_cA = (float)s.cA; s.f_cB = (float)s.cB;
     s.f_K0 = (float)s.K0; s.f_K1 = (float)s.K1; s.f_K2 = (float)s.K2;
-    s.f_K3 = (float)s.K3; s.f_K4 = (float)s.K3; s.f_hdt = (float)s.hdt;
+    s.f_K3 = s.f_K4 = (float)K3; s.f_hdt = (float)s.hdt;
     s.f_c = (float)(0.5 * dt * (p.kappa * p.rho / p.sigma - 0.5));
     ds_split(s.disc, s.ds_disc);
     ds_split(p.theta * (1.0 - s.disc), s.ds_m0);

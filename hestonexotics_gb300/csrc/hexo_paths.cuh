@@ -58,7 +58,7 @@ __device__ __forceinline__ bool qe_step(PathVars<false> &pv, const SegDesc &sg, 
     const double m = __fma_rn(v, sg.disc, sg.m0);                            // tpp:59
     const double s2 = fabs(__fma_rn(v, sg.cA, sg.cB));                       // tpp:60
     const bool near = f64::in_range(m, s2);
-    const bool quad = near ? f64::quadratic(m, s2) : s2 < __dmul_rn(1.5, __dmul_rn(m, m));
+    const bool quad = f64::quadratic(m, s2, near);
     if (dev::draw_prepare<false>(g, c, r, ws, quad)) dp = dev::draw_prefetch(c, r);
     float z1 = 0.0f, z2;                                                     // draw order, tpp:67,72,80
     uint64_t uw = 0;
@@ -68,9 +68,9 @@ __device__ __forceinline__ bool qe_step(PathVars<false> &pv, const SegDesc &sg, 
     else if (quad) vn = f64::variance_quadratic(m, s2, z1);                  // tpp:64-68
     else vn = f64::variance_exponential(m, s2, uw);                          // tpp:70-73
     pv.v = vn;
-    const double sd = f64::root(__dmul_rn(sg.K3, __dadd_rn(v, vn)));
-    const double t = __fma_rn(sg.K2, vn, __fma_rn(sg.K1, v, __dadd_rn(pv.lx, sg.K0)));   // tpp:80
-    pv.lx = __fma_rn(sd, f64::to_double(z2), t);
+    // tpp:80, sqrt(K3 v + K4 vn) z as sqrt(v + vn) (z sqrt(K3))
+    const double t = __fma_rn(sg.K2, vn, __fma_rn(sg.K1, v, __dadd_rn(pv.lx, sg.K0)));
+    pv.lx = __fma_rn(f64::root(__dadd_rn(v, vn)), f64::mul_float(z2, sg.rK3), t);
     pv.Xp = pv.X;
     pv.X = f64::exp_tab(pv.lx, etab);                                        // tpp:82
     return quad;

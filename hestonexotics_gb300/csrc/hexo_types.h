@@ -52,7 +52,8 @@ struct SegDesc {
     double disc;    // exp(-kappa dt)
     double cA;      // sigma^2 disc / kappa (1 - disc)
     double cB;      // theta sigma^2 / (2 kappa) (1 - disc)^2
-    double K0, K1, K2, K3;      // K0 includes (r - q) dt; the reference's K4 equals K3
+    double K0, K1, K2;          // K0 includes (r - q) dt
+    double rK3;     // sqrt(K3), the reference's K3 and K4 being equal (at least 2^-200: |rho| = 1 makes them 0)
     double m0;      // theta (1 - disc): m = v disc + m0
     double hdt;       // 0.5 dt: trapezoid weight after a non-pricing step
     double hdt_after; // 0.5 dt of the next segment: trapezoid weight after the pricing step
