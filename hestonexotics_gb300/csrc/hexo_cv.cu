@@ -26,6 +26,7 @@
 #include <vector>
 #include "hexo_plan.h"
 #include "hexo_launch.h"
+#include "hexo_f64.cuh"
 
 namespace hexo {
 
@@ -56,42 +57,107 @@ __device__ __forceinline__ cd cadd(cd a, cd b) { return {a.x + b.x, a.y + b.y}; 
 __device__ __forceinline__ cd csub(cd a, cd b) { return {a.x - b.x, a.y - b.y}; }
 __device__ __forceinline__ cd cmul(cd a, cd b) { return {a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x}; }
 __device__ __forceinline__ cd cscale(cd a, double s) { return {a.x * s, a.y * s}; }
-__device__ __forceinline__ cd cdiv(cd a, cd b) {   // one FP64 division (slow on this GPU) per quotient
-    const double d = 1.0 / (b.x * b.x + b.y * b.y);
+__device__ __forceinline__ cd cdiv(cd a, cd b) {
+    const double d = f64::recip_any(b.x * b.x + b.y * b.y);
     return {(a.x * b.x + a.y * b.y) * d, (a.y * b.x - a.x * b.y) * d};
 }
 __device__ __forceinline__ cd cexp(cd a) {
     double s, c;
-    sincos(a.y, &s, &c);
-    const double e = exp(a.x);
+    f64::sincos_tab(a.y, &s, &c);
+    const double e = f64::exp_tab(a.x, &f64::kExpTabInit);
     return {e * c, e * s};
 }
-__device__ __forceinline__ cd clog(cd a) { return {log(hypot(a.x, a.y)), atan2(a.y, a.x)}; }
+__device__ __forceinline__ cd clog(cd a) { return {0.5 * log(a.x * a.x + a.y * a.y), atan2(a.y, a.x)}; }
 __device__ __forceinline__ cd csqrt(cd a) {   // principal branch
-    const double r = hypot(a.x, a.y);
-    if (r == 0.0) return {0.0, 0.0};
-    const double t = sqrt(0.5 * (r + fabs(a.x)));
-    return a.x >= 0.0 ? cd{t, a.y / (2.0 * t)} : cd{fabs(a.y) / (2.0 * t), copysign(t, a.y)};
+    const double r = f64::root_any(a.x * a.x + a.y * a.y);
+    if (__double_as_longlong(r) == 0) return {0.0, 0.0};
+    const double t = f64::root_any(0.5 * (r + fabs(a.x))), h = 0.5 * fabs(a.y) * f64::recip_any(t);
+    return __double2hiint(a.x) >= 0 ? cd{t, copysign(h, a.y)} : cd{h, copysign(t, a.y)};
 }
 
-// The Heston affine solution over tau with terminal exponent b:
-// E_t[exp(a (y_T - y_t) + b v_T)] = exp(A + B v_t) ("little trap" form).
-__device__ __forceinline__ void heston_affine(cd a, cd b, double tau, const CvMat &m, cd &A, cd &B) {
-    const double s2 = m.sigma * m.sigma;
-    const cd beta = {m.kappa - m.rho * m.sigma * a.x, -m.rho * m.sigma * a.y};
-    const cd am1 = {a.x - 1.0, a.y};
-    cd D = csqrt(csub(cmul(beta, beta), cscale(cmul(a, am1), s2)));
-    if (D.x < 0.0) D = {-D.x, -D.y};
-    const cd s2b = cscale(b, s2);
-    const cd g = cdiv(csub(csub(beta, D), s2b), csub(cadd(beta, D), s2b));
+// One step of the Heston affine solution, E_t[exp(a (y_T - y_t) + b v_T)] =
+// exp(A + B v_t) over tau.  B is a Moebius map of the terminal exponent b:
+// with beta = kappa - rho sigma a, D = sqrt(beta^2 - s2 a (a - 1)), e = e^{-D tau},
+//   B(b) = (M00 b + M01) / (M10 b + M11),
+//   M = [[(beta + D) e - (beta - D), a (a - 1) (1 - e)], [s2 (e - 1), (beta + D) - (beta - D) e]] / (2 D)
+// ((beta - D)(beta + D) = s2 a (a - 1) by the definition of D), and
+//   A = a mu tau + kappa theta / s2 ((beta - D) tau - 2 log(M10 b + M11)):
+// the "little trap" form's logarithm (1 - g e) / (1 - g) is that denominator.
+// So b goes along as x / y with (x, y) <- M (x, y), y collects the product of
+// the denominators, and its logarithm is taken once for several steps instead
+// of a complex logarithm and three quotients for each.
+struct AffineStep {
+    cd M[4];
+    cd dA;      // the part of A without the logarithm
+};
+__device__ __forceinline__ void affine_step(cd a, double tau, const CvMat &m, AffineStep &s) {
+    const double s2 = m.sigma * m.sigma, rs = m.rho * m.sigma;
+    const cd beta = {m.kappa - rs * a.x, -rs * a.y};
+    const cd aam1 = {a.x * (a.x - 1.0) - a.y * a.y, a.y * (2.0 * a.x - 1.0)};
+    const cd D = csqrt(csub(cmul(beta, beta), cscale(aam1, s2)));
     const cd e = cexp(cscale(D, -tau));
-    const cd ge = cmul(g, e);
-    const cd one_ge = {1.0 - ge.x, -ge.y};
-    B = cdiv(csub(csub(beta, D), cmul(cadd(beta, D), ge)), cscale(one_ge, s2));
-    const cd lg = clog(cdiv(one_ge, cd{1.0 - g.x, -g.y}));
-    const cd inner = csub(cscale(csub(beta, D), tau), cscale(lg, 2.0));
-    A = cadd(cscale(a, m.mu * tau), cscale(inner, m.kappa * m.theta / s2));
+    const double d = f64::recip_any(D.x * D.x + D.y * D.y);
+    const cd h = {0.5 * D.x * d, -0.5 * D.y * d};              // 1 / (2 D)
+    const cd bpd = cmul(cadd(beta, D), h), bmd = csub(beta, D), bmh = cmul(bmd, h);
+    const cd om = cmul(cd{1.0 - e.x, -e.y}, h);
+    s.M[0] = csub(cmul(bpd, e), bmh);
+    s.M[1] = cmul(aam1, om);
+    s.M[2] = cscale(om, -s2);
+    s.M[3] = csub(bpd, cmul(bmh, e));
+    s.dA = cadd(cscale(a, m.mu * tau), cscale(bmd, m.kappa * m.theta / s2 * tau));
 }
+
+// A double to float accuracy, without the FP64 pipe's conversion: its leading
+// 20 bits (0 below 2^-126, infinite from 2^128 on).
+__device__ __forceinline__ float lead(double x) {
+    const uint32_t h = (uint32_t)__double2hiint(x), a = h & 0x7fffffffu;
+    const uint32_t b = a < 0x38100000u ? 0u : a >= 0x47f00000u ? 0x7f800000u : (a << 3) ^ 0x40000000u;
+    return __uint_as_float((b & 0x7fffffffu) | (h & 0x80000000u));
+}
+
+// A backward run of the recursion: b = x / y, the sum of A.  A step whose
+// denominator turns y by little (its quotient within 1/4 of 1, an argument
+// below 0.26) joins the product; the logarithms of up to 12 such are taken at
+// once, so that the sum of principal values stays what it is step by step.
+constexpr int kLogSteps = 12;
+struct AffineRun {
+    cd x, y, A;
+    int n;
+    __device__ __forceinline__ void start(cd b) {
+        x = b;
+        y = {1.0, 0.0};
+        A = {0.0, 0.0};
+        n = 0;
+    }
+    __device__ __forceinline__ void add_log(cd v, const CvMat &m) {
+        A = csub(A, cscale(clog(v), 2.0 * m.kappa * m.theta / (m.sigma * m.sigma)));
+    }
+    __device__ __forceinline__ void flush(const CvMat &m) {
+        add_log(y, m);
+        x = cdiv(x, y);
+        y = {1.0, 0.0};
+        n = 0;
+    }
+    __device__ __forceinline__ void step(const AffineStep &s, const CvMat &m) {
+        const cd nx = cadd(cmul(s.M[0], x), cmul(s.M[1], y)), ny = cadd(cmul(s.M[2], x), cmul(s.M[3], y));
+        const float yx = lead(y.x), yy = lead(y.y), dx = lead(ny.x) - yx, dy = lead(ny.y) - yy;
+        const bool little = dx * dx + dy * dy < 0x1.fp-5f * (yx * yx + yy * yy);   // false for infinities and NaN
+        if (!little && n > 0) add_log(y, m);
+        const cd y0 = y;
+        x = nx;
+        y = ny;
+        A = cadd(A, s.dA);
+        ++n;
+        if (!little) {   // this step's quotient by itself
+            add_log(n > 1 ? cdiv(ny, y0) : ny, m);
+            x = cdiv(x, y);
+            y = {1.0, 0.0};
+            n = 0;
+        } else if (n >= kLogSteps) {
+            flush(m);
+        }
+    }
+};
 
 // phi[m * (kCvNodes + 1) + i] = E[exp(z L)], z = 1/2 + i U x_i for the nodes
 // and z = 1 (E[G] / S0) at i = kCvNodes.
@@ -103,57 +169,47 @@ __global__ void cv_cf_kernel(const CvMat *__restrict__ mats, uint32_t mat0, uint
     const uint32_t mi = t / (kCvNodes + 1), i = t % (kCvNodes + 1);
     const CvMat m = mats[mi];
     const cd z = i == (uint32_t)kCvNodes ? cd{1.0, 0.0} : cd{0.5, m.U * nodes[i].x};
-    cd Asum = {0.0, 0.0}, b = {0.0, 0.0}, Th = {0.0, 0.0};
+    AffineRun run;
+    run.start(cd{0.0, 0.0});
+    double C = 0.0;
     for (uint32_t k = m.n_steps; k-- > 0;) {
         const double2 s = steps[m.step_begin + k];   // (dt, c)
-        Th = cadd(Th, cscale(z, s.y));
-        cd A, B;
-        heston_affine(Th, b, s.x, m, A, B);
-        Asum = cadd(Asum, A);
-        b = B;
+        C += s.y;
+        AffineStep as;
+        affine_step(cscale(z, C), s.x, m, as);
+        run.step(as, m);
     }
-    const cd r = cexp(cadd(Asum, cscale(b, m.v0)));
+    if (run.n > 0) run.flush(m);
+    const cd r = cexp(cadd(run.A, cscale(run.x, m.v0)));
     phi[t] = make_double2(r.x, r.y);
 }
 
 // The same recursion for one (maturity, node) per warp, for requests too
 // small to fill the GPU with one thread per pair (each SM's FP64 pipe then
-// serves a single warp that walks every grid step in turn).  Over a fixed
-// step, heston_affine's B is a Moebius map of the terminal exponent b:
-//   B(b) = (M00 b + M01) / (M10 b + M11),  e = exp(-D tau),
-//   M = [[(beta + D) e - (beta - D), a (a - 1) (1 - e)], [s2 (e - 1), (beta + D) - (beta - D) e]]
-// ((beta - D)(beta + D) = s2 a (a - 1) by the definition of D).  Lane l
-// takes a block of consecutive steps; one warp scan gives every block the
-// sum of the c_j after it and the product of the later blocks' maps, whose
-// value at b = 0 is the b entering the block's last step; the lane then runs
-// heston_affine backward over its own steps, exactly as the one-thread
-// kernel does, and the warp sums the A terms.
-__device__ __forceinline__ void mobius(cd a, double tau, const CvMat &m, cd (&M)[4]) {
-    const double s2 = m.sigma * m.sigma;
-    const cd beta = {m.kappa - m.rho * m.sigma * a.x, -m.rho * m.sigma * a.y};
-    const cd aam1 = cmul(a, cd{a.x - 1.0, a.y});
-    cd D = csqrt(csub(cmul(beta, beta), cscale(aam1, s2)));
-    if (D.x < 0.0) D = {-D.x, -D.y};
-    const cd e = cexp(cscale(D, -tau));
-    const cd bpd = cadd(beta, D), bmd = csub(beta, D);
-    M[0] = csub(cmul(bpd, e), bmd);
-    M[1] = cmul(aam1, cd{1.0 - e.x, -e.y});
-    M[2] = cscale(cd{e.x - 1.0, e.y}, s2);
-    M[3] = csub(bpd, cmul(bmd, e));
-}
-// X <- X Y, rescaled by a power of two (a Moebius map does not change when
-// its matrix is scaled, and the products of many steps would otherwise
-// drift out of range).
+// serves a single warp that walks every grid step in turn).  Lane l takes a
+// block of consecutive steps; one warp scan gives every block the sum of the
+// c_j after it and the product of the later blocks' maps, whose value at b = 0
+// is the b entering the block's last step; the lane then runs its own steps
+// backward, exactly as the one-thread kernel does, and the warp sums the A
+// terms.
+// X <- X Y
 __device__ __forceinline__ void mobius_mul(cd (&X)[4], const cd (&Y)[4]) {
     cd R[4];
     R[0] = cadd(cmul(X[0], Y[0]), cmul(X[1], Y[2]));
     R[1] = cadd(cmul(X[0], Y[1]), cmul(X[1], Y[3]));
     R[2] = cadd(cmul(X[2], Y[0]), cmul(X[3], Y[2]));
     R[3] = cadd(cmul(X[2], Y[1]), cmul(X[3], Y[3]));
-    double mx = 0.0;
-    for (int i = 0; i < 4; ++i) mx = fmax(mx, fmax(fabs(R[i].x), fabs(R[i].y)));
-    const int ex = mx > 0.0 ? ilogb(mx) : 0;
-    for (int i = 0; i < 4; ++i) X[i] = {scalbn(R[i].x, -ex), scalbn(R[i].y, -ex)};
+    for (int i = 0; i < 4; ++i) X[i] = R[i];
+}
+// X rescaled by a power of two (a Moebius map does not change when its matrix
+// is scaled, and the products of many steps would otherwise drift out of range).
+__device__ __forceinline__ void mobius_rescale(cd (&X)[4]) {
+    uint32_t e = 0;
+    for (int i = 0; i < 4; ++i)
+        e = max(e, max((uint32_t)__double2hiint(X[i].x) & 0x7ff00000u, (uint32_t)__double2hiint(X[i].y) & 0x7ff00000u));
+    if (e == 0u || e == 0x7ff00000u) return;
+    const double s = __hiloint2double((int)(0x7fe00000u - e), 0);   // 2^-exponent
+    for (int i = 0; i < 4; ++i) X[i] = cscale(X[i], s);
 }
 __device__ __forceinline__ cd shfl_down_cd(cd v, unsigned d) {
     return {__shfl_down_sync(0xffffffffu, v.x, d), __shfl_down_sync(0xffffffffu, v.y, d)};
@@ -179,41 +235,44 @@ __global__ void cv_cf_warp_kernel(const CvMat *__restrict__ mats, uint32_t n_mat
     }
     double c_after = __shfl_down_sync(0xffffffffu, cs, 1);
     if (lane == 31u) c_after = 0.0;
-    cd P[4] = {{1.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {1.0, 0.0}};
+    cd S[4] = {{1.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {1.0, 0.0}};
     {
         double C = c_after;
-        cd Mk[4];
-        for (uint32_t k = k1; k-- > k0;) {   // P = M_k0 ... M_(k1-1)
+        AffineStep as;
+        for (uint32_t k = k1; k-- > k0;) {   // S = M_k0 ... M_(k1-1)
             C += st[k].y;
-            mobius(cscale(z, C), st[k].x, m, Mk);
-            cd T[4] = {Mk[0], Mk[1], Mk[2], Mk[3]};
-            mobius_mul(T, P);
-            for (int q = 0; q < 4; ++q) P[q] = T[q];
+            affine_step(cscale(z, C), st[k].x, m, as);
+            mobius_mul(as.M, S);
+            for (int q = 0; q < 4; ++q) S[q] = as.M[q];
+            if (((k1 - k) & 7u) == 0u) mobius_rescale(S);
         }
+        mobius_rescale(S);
     }
     // the later blocks' maps: an inclusive suffix product, then shifted by one lane
-    cd S[4] = {P[0], P[1], P[2], P[3]};
     for (unsigned d = 1; d < 32u; d <<= 1) {
         cd X[4];
         for (int q = 0; q < 4; ++q) X[q] = shfl_down_cd(S[q], d);
-        if (lane + d < 32u) mobius_mul(S, X);
+        if (lane + d < 32u) {
+            mobius_mul(S, X);
+            mobius_rescale(S);
+        }
     }
-    cd N[4];
-    for (int q = 0; q < 4; ++q) N[q] = shfl_down_cd(S[q], 1);
-    cd b = lane == 31u ? cd{0.0, 0.0} : cdiv(N[1], N[3]);   // the later blocks' map at b = 0
-    // this block's steps, backward, as the one-thread recursion runs them
-    cd Asum = {0.0, 0.0};
+    const cd N1 = shfl_down_cd(S[1], 1), N3 = shfl_down_cd(S[3], 1);
+    // this block's steps, backward from the later blocks' map at b = 0, as the one-thread recursion runs them
+    AffineRun run;
+    run.start(lane == 31u ? cd{0.0, 0.0} : cdiv(N1, N3));
     double C = c_after;
     for (uint32_t k = k1; k-- > k0;) {
         C += st[k].y;
-        cd A, B;
-        heston_affine(cscale(z, C), b, st[k].x, m, A, B);
-        Asum = cadd(Asum, A);
-        b = B;
+        AffineStep as;
+        affine_step(cscale(z, C), st[k].x, m, as);
+        run.step(as, m);
     }
+    if (run.n > 0) run.flush(m);
+    cd Asum = run.A;
     for (unsigned d = 16; d > 0u; d >>= 1) Asum = cadd(Asum, shfl_down_cd(Asum, d));
     if (lane == 0u) {   // lane 0's block is the first: its b is b_0
-        const cd r = cexp(cadd(Asum, cscale(b, m.v0)));
+        const cd r = cexp(cadd(Asum, cscale(run.x, m.v0)));
         phi[t] = make_double2(r.x, r.y);
     }
 }

@@ -169,6 +169,28 @@ constexpr LogTab make_log_tab() {
     }
     return r;
 }
+constexpr int kTurnTab = 256;  // sin and cos of 2 pi j / 256
+struct TurnTab {
+    double s[kTurnTab], c[kTurnTab];
+};
+constexpr DD kPi = {0x1.921fb54442d18p+1, 0x1.1a62633145c07p-53};
+constexpr TurnTab make_turn_tab() {
+    TurnTab r{};
+    for (int j = 0; j < kTurnTab; ++j) {   // Taylor series at the angle within (-pi, pi]
+        const DD x = dd_mul(kPi, DD{(j <= kTurnTab / 2 ? j : j - kTurnTab) * (2.0 / kTurnTab), 0.0});
+        DD s{0.0, 0.0}, c{0.0, 0.0}, t{1.0, 0.0};
+        for (int n = 0; n < 48; n += 2) {
+            c = dd_add(c, t);
+            t = dd_div(dd_mul(t, x), DD{n + 1.0, 0.0});
+            s = dd_add(s, t);
+            t = dd_div(dd_mul(t, x), DD{-(n + 2.0), 0.0});
+        }
+        r.s[j] = s.h;
+        r.c[j] = c.h;
+    }
+    return r;
+}
+__device__ constexpr TurnTab kTurnTabDev = make_turn_tab();
 __device__ constexpr ExpTab kExpTabInit = make_exp_tab();
 __device__ constexpr LogTab kLogTabDev = make_log_tab();
 
@@ -214,6 +236,27 @@ __device__ __forceinline__ double exp_tab(double x, const ExpTab *tab) {
     const uint32_t s = hi(y) >> 31;        // 2^63 or more: the next binade
     y >>= s;
     return __longlong_as_double((long long)(((uint64_t)(1022u + (uint32_t)(n >> 8) + s) << 52) + ((y + 512ull) >> 10)));
+}
+
+// sin(x) and cos(x), within 1.3 ulp of 1: x = n 2 pi / 256 + d, |d| <= pi /
+// 256, the table's sine and cosine turned by d (sin d to d^5, cos d - 1 to
+// d^6).  15 FP64 instructions (the library's sincos: about 45).
+__device__ __forceinline__ void sincos_tab(double x, double *sn, double *cs) {
+    if ((hi32(x) & 0x7fffffffu) >= 0x41600000u) {   // |x| >= 2^23, infinite or NaN
+        sincos(x, sn, cs);
+        return;
+    }
+    constexpr double H = kPi.h / (kTurnTab / 2), L = kPi.l / (kTurnTab / 2);
+    const double t = __fma_rn(x, 1.0 / H, 0x1.8p52), n = __dsub_rn(t, 0x1.8p52);
+    const uint32_t j = lo32(t) & (uint32_t)(kTurnTab - 1);
+    const double d = __fma_rn(-n, L, __fma_rn(-n, H, x)), d2 = __dmul_rn(d, d);
+    const float f2 = __double2float_rn(d2);
+    const double q = __dadd_rn(-1.0 / 6.0, to_double(__fmul_rn(f2, 1.0f / 120.0f)));
+    const double s = __fma_rn(__dmul_rn(d, d2), q, d);                                        // sin d
+    const double u = __dmul_rn(d2, __dadd_rn(-0.5, to_double(__fmul_rn(f2, __fmaf_rn(f2, -1.0f / 720.0f, 1.0f / 24.0f)))));
+    const double s0 = kTurnTabDev.s[j], c0 = kTurnTabDev.c[j];
+    *sn = __fma_rn(c0, s, __fma_rn(s0, u, s0));
+    *cs = __fma_rn(-s0, s, __fma_rn(c0, u, c0));
 }
 
 // -log(x) in units of 2^-57 of x = P 2^(k-63), 2^63 <= P < 2^64, -80 < k < 0,
@@ -274,6 +317,16 @@ __device__ __forceinline__ double recip(double x) {
     const float unit = __uint_as_float(0x7f000000u + (52u << 23) - (__float_as_uint(y.h) & 0x7f800000u));
     const int32_t k = __float2int_rn(__fmul_rn(__fmul_rn(remainder_mul(1.0, x, Y), r), unit));
     return __longlong_as_double(__double_as_longlong(Y) + (long long)k);
+}
+
+// The same for any x > 0, and sqrt(x) for any x >= 0 (the ranges [2^-60, 2^60)
+// and [2^-60, 2^100) tested on the exponent: a comparison is an FP64
+// instruction too).
+__device__ __forceinline__ double recip_any(double x) {
+    return hi32(x) - 0x3c300000u < 0x07800000u ? recip(x) : 1.0 / x;
+}
+__device__ __forceinline__ double root_any(double x) {
+    return hi32(x) - 0x3c300000u < 0x0a000000u ? root(x) : sqrt(x);
 }
 
 // x / y from r = 1 / y rounded (0: not given): the product corrected by its
@@ -362,27 +415,25 @@ __device__ __forceinline__ double variance_exponential(double m, double s2, uint
     e = __fmaf_rn(-y0, Mf.l, __fadd_rn(e, Wf.l));
     const ds::F2 Yf = ds::fast_two_sum(y0, __fmul_rn(e, rm));
     const uint64_t N = 0ull - uw;                                     // 1 - U = N 2^-64 (uw == 0: U = 0 < p)
-    if (N == 0ull) return 0.0;
     const double Y = join(Yf);
     // x = Y (1 - U) = P 2^(k-63)
     const uint64_t Ym = (uint64_t)__double_as_longlong(Y) << 11 | 0x8000000000000000ull;
-    const int lz = __clzll((long long)N);
+    const int lz = __clzll((long long)N) & 63;
     uint64_t P = mul_hi(Ym, N << lz);
     const int s = (int)(~hi(P) >> 31), eY = (int)(hi32(Y) >> 20) - 1023;
     const int k = eY - lz - s;
-    if (k >= 0) return 0.0;                                           // p >= U
     P <<= s;
     const float d = __fdividef(__fmul_rn(remainder_mul(W, Y, mm2), rm), y0);
     // m Y (-log x), its significand in 64 bits
-    uint64_t A = neg_log_fixed(P, k, d);
-    if (A == 0ull) return 0.0;
-    const int la = __clzll((long long)A);
+    const uint64_t A = neg_log_fixed(P, k, d);
+    const int la = __clzll((long long)A) & 63;
     uint64_t V = mul_hi((uint64_t)__double_as_longlong(m) << 11 | 0x8000000000000000ull, Ym);   // 2^61.99 or more
     V = mul_hi(V, A << la);
-    const int lv = __clzll((long long)V);
+    const int lv = __clzll((long long)V) & 63;
     V <<= lv;
     const uint32_t ev = (hi32(m) >> 20) + (uint32_t)(eY + 8 - la - lv);   // the leading bit's exponent
-    return __longlong_as_double((long long)(((uint64_t)(ev - 1u) << 52) + ((V + 1024ull) >> 11)));
+    const double v = __longlong_as_double((long long)(((uint64_t)(ev - 1u) << 52) + ((V + 1024ull) >> 11)));
+    return N != 0ull && k < 0 && A != 0ull ? v : 0.0;                 // k >= 0: p >= U
 }
 
 // The next variance outside in_range, in the reference's order of operations.
