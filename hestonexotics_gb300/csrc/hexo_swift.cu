@@ -161,19 +161,16 @@ __host__ __device__ inline void chf_grad_reference(const HP &p, double tau, cplx
 //   A = v0 f T / Q, D = log(2 d / ((1 + E) Q)) + (kappa - d) tau / 2, E = e^{-d tau},
 //   a2r = A2_rho / A2 = W (2 + xi tau) (xi + d T) / (2 d Q),  W = i sigma u,
 //   A_rho = fv d_rho - A a2r,  fv = v0 tau f / (2 Q),  d_rho = xi W / d, and so on.
-// T = (1 - |E|^2 - 2 i Im E) / |1 + E|^2 from expm1 keeps its accuracy for
-// small d tau.  One exp, one expm1, two sincos, one log, one atan2 and about
-// 45 complex products: some 350 FP64 instructions, against 1,400 with the
+// With T = (1 - E) / (1 + E) everything stands over (1 + E) Q = 2 d - (d - xi)
+// (1 - E); 1 - E comes from expm1 and half angles, d - xi from sigma^2 f / (d +
+// xi) and the logarithm from log1p, so nothing cancels at low frequencies,
+// where D goes to 0 and most of a price comes from.  One exp, one expm1, two
+// sincos, one log1p, one atan2 and about 45 complex products: some 320 FP64
+// instructions, against 1,400 with the
 // two dozen complex quotients of the reference's form.  False, for that form,
 // from d tau / 2 = 300 on, where sinh, cosh and the squares of A2 come near the
 // end of the double range: what it gives there (phi is below e^{-300}, and
 // beyond the range the result is NaN) is what it gave before.
-__device__ __forceinline__ double recip(double x) {   // 1 / x, x > 0
-    return x > 0x1p-60 && x < 0x1p60 ? f64::recip(x) : 1.0 / x;
-}
-__device__ __forceinline__ double sqroot(double x) {   // sqrt(x), x >= 0
-    return x > 0x1p-100 && x < 0x1p100 ? f64::root(x) : sqrt(x);
-}
 __device__ __forceinline__ double norm(cplx a) { return a.re * a.re + a.im * a.im; }
 __device__ __forceinline__ cplx conj(cplx a) { return C(a.re, -a.im); }
 
@@ -186,38 +183,40 @@ __device__ __forceinline__ bool chf_grad(const HP &p, const ChfConst &q, double 
     const cplx xi = C(p.kappa, su * p.rho), f = C(u * u, -u);
     // d = sqrt(xi^2 + sigma^2 f), principal
     const cplx d2 = C(xi.re * xi.re - xi.im * xi.im + su * su, 2.0 * xi.re * xi.im - p.sigma * su);
-    const double r = sqroot(norm(d2)), t0 = sqroot(0.5 * (r + fabs(d2.re))), t1 = 0.5 * fabs(d2.im) * recip(t0);
-    const cplx d = C(d2.re >= 0.0 ? t0 : t1, copysign(d2.re >= 0.0 ? t1 : t0, d2.im));
+    const double r = f64::root_any(norm(d2)), t0 = f64::root_any(0.5 * (r + fabs(d2.re))), t1 = 0.5 * fabs(d2.im) * f64::recip_any(t0);
+    const bool right = __double2hiint(d2.re) >= 0;
+    const cplx d = C(right ? t0 : t1, copysign(right ? t1 : t0, d2.im));
     if (!(d.re * tau < 600.0) || p.v0 < 1e-12) return false;
-    double sn, cs;
-    sincos(d.im * tau, &sn, &cs);
-    const double em = expm1(-(d.re * tau)), a = 1.0 + em;   // E = a (cs - i sn)
-    const double iden = recip(1.0 + a * (2.0 * cs + a));    // 1 / |1 + E|^2
-    const cplx T = C(-em * (2.0 + em) * iden, 2.0 * a * sn * iden);
-    const cplx Q = d + xi * T;
-    const cplx iQ = conj(Q) * recip(norm(Q)), id = conj(d) * recip(norm(d));
-    const cplx fq = f * iQ, A = p.v0 * (fq * T);
-    const cplx z = (2.0 * iden) * (d * C(1.0 + a * cs, a * sn)) * iQ;
-    const cplx D = C(0.5 * log(norm(z)) + (p.kappa - d.re) * (0.5 * tau), atan2(z.im, z.re) - d.im * (0.5 * tau));
+    // E = e^{-d tau}: 1 - E and 1 + E without cancellation, from expm1 and the half angle
+    double hs, hc;
+    f64::sincos_tab(0.5 * (d.im * tau), &hs, &hc);
+    const double em = expm1(-(d.re * tau)), a = 1.0 + em, v = 2.0 * hs * hs, sn = a * (2.0 * hs * hc);
+    const cplx oE = C(a * v - em, sn), pE = C(1.0 + a * (1.0 - v), -sn);
+    const cplx dp = d + xi, dm = (p.sigma * p.sigma * f64::recip_any(norm(dp))) * (f * conj(dp));   // d - xi = sigma^2 f / (d + xi)
+    const cplx dE = dm * oE, zd = 2.0 * d - dE;              // (1 + E) Q
+    const cplx iz = conj(zd) * f64::recip_any(norm(zd)), id = conj(d) * f64::recip_any(norm(d));
+    const cplx fz = f * iz, fq = fz * pE, fT = fz * oE;      // f / Q and f T / Q
+    const cplx A = p.v0 * fT, w = dE * iz;                   // 1 + w = 2 d / ((1 + E) Q)
+    const cplx D = C(0.5 * (log1p(2.0 * w.re + norm(w)) - tau * dm.re), atan2(w.im, 1.0 + w.re) - 0.5 * tau * (dm.im + xi.im));
     const double vt = p.vm * tau * u * q.is;   // t = vm tau i u / sigma
     const double er = q.k2 * D.re - A.re, ei = p.kappa * p.rho * vt + q.k2 * D.im - A.im;
     double ps, pc;
-    sincos(ei, &ps, &pc);
+    f64::sincos_tab(ei, &ps, &pc);
     const double ea = f64::exp_tab(er, &f64::kExpTabInit);
     const cplx c = C(ea * pc, ea * ps);
     const cplx W = C(0.0, su), h = C(2.0 + xi.re * tau, xi.im * tau);
     const cplx xw = xi * W, d_rho = xw * id;
-    const cplx a2r = (0.5 * (W * h)) * ((xi + d * T) * (id * iQ));
+    const cplx a2r = (0.5 * (W * h)) * id * ((xi * pE + d * oE) * iz);
     const cplx fv = (0.5 * tau * p.v0) * fq;
     const cplx A_rho = fv * d_rho - A * a2r;
     const cplx br = d_rho * id - a2r;                        // B_rho / B
     const cplx d_sigma = (q.rs * xw - W + su * u) * id;
-    const cplx a2s = q.rs * a2r + (0.5 * p.sigma) * (fq * (h * id + tau * T));
+    const cplx a2s = q.rs * a2r + (0.5 * p.sigma) * (fq * (h * id) + tau * fT);
     const cplx A_sigma = fv * d_sigma - A * a2s;
     const double iw = -q.is / u;                              // 1 / W = i iw
     const cplx i_br = C(-iw * br.im, iw * br.re), i_ar = C(-iw * A_rho.im, iw * A_rho.re);
     out[0] = c;
-    out[1] = -(c * (fq * T));
+    out[1] = -(c * fT);
     out[2] = c * ((2.0 * p.kappa * q.is * q.is) * D + C(0.0, p.kappa * p.rho * tau * u * q.is));
     out[3] = c * (q.k2 * br - A_rho + C(0.0, vt * p.kappa));
     out[4] = c * (q.k2 * (i_br + 0.5 * tau) - i_ar + (2.0 * p.vm * q.is * q.is) * D + C(0.0, vt * p.rho));
@@ -579,7 +578,7 @@ __global__ void __launch_bounds__(64) density_kernel(const Exp *ex, const Item *
 // One warp per option: Re sum_j W_q(j) disc K e^{-i u_j x}.  A lane's terms
 // are 32 j apart, so its phase turns by e^{-i 64 du x} from one to the next:
 // one complex product instead of a sincos (4 FP64 instructions instead of
-// about 45), and a sincos every 16 terms, so that the products' roundings do
+// a sincos's 45, or 15 by table), and a sincos every 16 terms, so that the products' roundings do
 // not add up beyond the sincos argument's own.  kGrad: the gradient too.
 constexpr uint32_t kTurns = 16;
 template <bool kGrad>
@@ -593,8 +592,9 @@ __global__ void __launch_bounds__(128) price_kernel(const Exp *ex, const Item *i
     double acc[6] = {0, 0, 0, 0, 0, 0};
     const uint32_t span = 32u * (E.stiff ? 1u : kTurns);
     for (uint32_t j0 = lane; j0 < E.J; j0 += span) {
-        double s, c;
-        sincos((2.0 * j0 + 1.0) * E.du * o.x, &s, &c);     // e^{-i u x} = c - i s
+        double s, c;     // e^{-i u x} = c - i s
+        if (E.stiff) sincos((2.0 * j0 + 1.0) * E.du * o.x, &s, &c);
+        else f64::sincos_tab((2.0 * j0 + 1.0) * E.du * o.x, &s, &c);
         const uint32_t j1 = min(E.J, j0 + span);
         for (uint32_t j = j0; j < j1; j += 32) {
 #pragma unroll
