@@ -46,22 +46,64 @@ LaunchShape ctx_shape(hexo_ctx *ctx, const hexo_mc_cfg &cfg) {
     return sh;
 }
 
+namespace {
+// Whether the launch shape is the engine's to choose: the default, not an
+// explicit or tuned one.  The launch shape does not change results.
+bool shape_is_free(hexo_ctx *ctx, const hexo_mc_cfg &cfg, const LaunchShape &sh) {
+    const LaunchShape def{256, 1, 1};
+    const LaunchShape &tuned = cfg.precision == HEXO_FP32 ? ctx->shape_f32 : ctx->shape_f64;
+    return !cfg.block && !cfg.paths_per_thread && !cfg.unroll && sh.block == def.block && sh.ppt == def.ppt &&
+           tuned.block == def.block && tuned.ppt == def.ppt && tuned.unroll == def.unroll;
+}
+
+// Time of `ctas` CTAs of `block` threads a SM, in units of a full SM's (16
+// warps, four a scheduler): what is left of the latency when a scheduler has
+// one, two, three or four warps (measured, 126 steps: FP64 0.252, 0.284,
+// 0.345, 0.396 ms, FP32 0.113, 0.131, 0.160, 0.192 ms).
+double round_cost(uint32_t ctas, uint32_t block) {
+    constexpr double kTime[5] = {0.0, 0.61, 0.70, 0.85, 1.0};
+    return kTime[std::min(4u, (ctas * (block / 32u) + 3u) / 4u)];
+}
+
+// CTA width for one set whose paths all run the whole schedule: its equal
+// tiles go through the SMs in rounds, and a last round that few CTAs fill
+// costs nearly a whole one.  The width is the one whose full rounds and rest
+// take least by round_cost, narrower widths having finer rests and, at 96 and
+// 224 threads, nearly as many warps a SM.  Measured against 256 throughout
+// (plain Asian, 126 steps, FP64 / FP32): 80,000 paths 0.630 / 0.270 against
+// 0.698 / 0.287 ms at 192, 131,072 paths 0.779 / 0.348 against 0.859 / 0.369 at
+// 96, 200,000 paths 1.193 / 0.524 against 1.277 / 0.546 at 96; from 2^18 paths
+// on 256 is mostly best.  Uneven sets keep 256: their tiles are taken longest
+// first and fill the last round by themselves (nine books: 256 best in all).
+uint32_t uniform_block(hexo_ctx *ctx, uint64_t paths) {
+    uint32_t best = 256;
+    double best_cost = 1e300;
+    for (uint32_t b : {224u, 256u, 192u, 128u, 160u, 96u}) {
+        const uint64_t fit = ctx->smem_sm / (paths_smem_bytes(b, 1) + 1024u);   // 1 KB of the system's a CTA
+        const uint64_t ctas = std::min<uint64_t>(fit, 512u / b);                // 16 warps by registers
+        if (ctas == 0) continue;
+        const uint64_t tiles = (paths + b - 1) / b, slots = ctas * ctx->sm_count, rest = tiles % slots;
+        const double cost = (double)(tiles / slots) * round_cost((uint32_t)ctas, b) +
+                            round_cost((uint32_t)((rest + ctx->sm_count - 1) / ctx->sm_count), b);
+        if (cost < best_cost * 0.97) {   // the estimate is good to a few percent: an earlier width stands
+            best_cost = cost;
+            best = b;
+        }
+    }
+    return best;
+}
+} // namespace
+
 // A batch with fewer paths than the default shape's CTA slots (2 per SM of
 // 256 threads, one path each) would leave SMs with one CTA and others with
 // two; with narrower CTAs (a multiple of 32 threads, at least 128) the same
 // paths spread over every slot, so the most loaded SM runs fewer warps.
-// Only the default shape is changed (not an explicit or tuned one); the
-// launch shape does not change results.
 void fit_small_batch(hexo_ctx *ctx, const hexo_mc_cfg &cfg, LaunchShape &sh, const std::vector<SetPlan> &plans) {
-    const LaunchShape def{256, 1, 1};
-    const LaunchShape &tuned = cfg.precision == HEXO_FP32 ? ctx->shape_f32 : ctx->shape_f64;
-    if (cfg.block || cfg.paths_per_thread || cfg.unroll || sh.block != def.block || sh.ppt != def.ppt ||
-        tuned.block != def.block || tuned.ppt != def.ppt || tuned.unroll != def.unroll)
-        return;
+    if (!shape_is_free(ctx, cfg, sh)) return;
     uint64_t paths = 0;
     for (const SetPlan &sp : plans) paths += sp.path_hi - sp.path_lo;
     const uint64_t slots = (uint64_t)ctx->sm_count * 2;
-    if (paths == 0 || paths >= slots * def.block) return;
+    if (paths == 0 || paths >= slots * sh.block) return;
     const uint64_t per = (paths + slots - 1) / slots;
     sh.block = (uint32_t)std::max<uint64_t>(128, (per + 31) / 32 * 32);
 }
@@ -294,7 +336,12 @@ hexo_status plan_requests(hexo_ctx *ctx, const hexo_request *reqs, uint32_t n_re
         cv_base += 2u * plans[r].n_cv;
     }
     bp.shape = ctx_shape(ctx, cfg);
-    fit_small_batch(ctx, cfg, bp.shape, plans);
+    const SetPlan &first = plans[0];
+    if (n_reqs == 1 && first.path_hi > first.path_lo && first.thr[first.mats.size() - 1] >= first.path_hi &&
+        shape_is_free(ctx, cfg, bp.shape))
+        bp.shape.block = uniform_block(ctx, first.path_hi - first.path_lo);   // every path reaches the last maturity
+    else
+        fit_small_batch(ctx, cfg, bp.shape, plans);
     batch_tiles(bp, plans);
     return HEXO_OK;
 }
@@ -363,6 +410,8 @@ hexo_status hexo_ctx_create(hexo_ctx **out, const hexo_ctx_opts *opts) {
     ctx->sm_count = (uint32_t)v;
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
     ctx->smem_optin = (size_t)v;
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device);
+    ctx->smem_sm = (size_t)v;
     if (e != cudaSuccess) {
         delete ctx;
         return e == cudaErrorMemoryAllocation ? HEXO_ERR_NOMEM : HEXO_ERR_CUDA;

@@ -70,7 +70,7 @@ struct hexo_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     uint32_t sm_count = 0;
-    size_t smem_optin = 0;
+    size_t smem_optin = 0, smem_sm = 0;       // shared memory a CTA and a SM can have
     uint64_t mem_cap = 0;
     std::string tune_cache;
     hexo::LaunchShape shape_f64, shape_f32;   // tuned or default launch shapes
