@@ -25,10 +25,15 @@
 namespace hexo {
 
 
-// Square root of max(x, 0) from the MUFU reciprocal square root.
-__device__ __forceinline__ float fsqrt_fast(float x) {
-    const float y = fmaxf(x, 0.0f);
-    return __fmul_rn(y, rsqrtf(fmaxf(y, 1e-30f)));
+// Square root of x >= 0 from the MUFU reciprocal square root (the .ftz form:
+// its operand is normal, and the other form spends three instructions on
+// operands that are not).
+__device__ __forceinline__ float fsqrt_fast(float x) { return __fmul_rn(x, ds::rsqrt_approx(fmaxf(x, 1e-30f))); }
+// exp(x) as __expf, results below 2^-126 as 0.
+__device__ __forceinline__ float exp_fast(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__fmul_rn(x, 1.4426950408889634f)));
+    return r;
 }
 
 template <bool kF32> struct Real;
@@ -162,7 +167,7 @@ __device__ __forceinline__ bool qe_step(PathVars<true> &pv, const SegDesc &sg, d
     inc = __fmaf_rn(fsqrt_fast(__fmaf_rn(sg.f_K3, v.h, __fmul_rn(sg.f_K4, vn.h))), z2, inc);
     pv.lx = __fadd_rn(pv.lx, inc);
     pv.Xp = pv.X;
-    pv.X = __fmul_rn(S0, __expf(__fmaf_rn(rr, vn.h, pv.lx)));
+    pv.X = __fmul_rn(S0, exp_fast(__fmaf_rn(rr, vn.h, pv.lx)));
     return quad;
 }
 
