@@ -416,6 +416,10 @@ hexo_status hexo_ctx_create(hexo_ctx **out, const hexo_ctx_opts *opts) {
         delete ctx;
         return e == cudaErrorMemoryAllocation ? HEXO_ERR_NOMEM : HEXO_ERR_CUDA;
     }
+    if (cudaMallocHost(&ctx->pinned_keep, 64) != cudaSuccess) {   // only a matter of speed
+        (void)cudaGetLastError();
+        ctx->pinned_keep = nullptr;
+    }
     tune_load(ctx);
     *out = ctx;
     return HEXO_OK;
@@ -430,6 +434,7 @@ hexo_status hexo_ctx_destroy(hexo_ctx *ctx) {
     }
     if (ctx->arena_d) cudaFree(ctx->arena_d);
     if (ctx->arena_h) cudaFreeHost(ctx->arena_h);
+    if (ctx->pinned_keep) cudaFreeHost(ctx->pinned_keep);
     delete ctx;
     return HEXO_OK;
 }

@@ -82,6 +82,11 @@ struct hexo_ctx {
     // so no device synchronisation, per call once the largest batch was seen
     void *arena_d = nullptr, *arena_h = nullptr;
     size_t arena_dcap = 0, arena_hcap = 0;
+    // a few pinned bytes of the context's own: while they are held, the driver
+    // keeps the block that small pinned allocations come from (a prepared
+    // batch's results), which otherwise is mapped and unmapped with each
+    // (measured: preparing a small batch 0.56 ms without, 0.46 ms with)
+    void *pinned_keep = nullptr;
 };
 
 struct hexo_batch {
