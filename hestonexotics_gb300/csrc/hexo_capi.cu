@@ -165,11 +165,16 @@ hexo_status batch_upload(hexo_ctx *ctx, BatchPlan &&plan, bool f32, DeviceBatch 
     const size_t o_pexp = take(n_out * sizeof(int32_t));
     const bool carried = db.carry != nullptr;   // the serving loop's split requests
     const size_t o_carry = take(carried ? n_out * sizeof(uint64_t) : 0);
+    // cleared together by each run: the sums and the control block (queue head, error flags,
+    // exponential-branch steps); copied back together: the control block and the outputs
     const size_t o_acc = take((size_t)db.n_slots * n_out * kLimbs * sizeof(unsigned long long));
-    const size_t o_acc_sum = take((size_t)n_out * kLimbs * sizeof(unsigned long long));
+    const size_t o_ctl = take(kCtlBytes);
     const size_t o_price = take(n_out * sizeof(double));
     const size_t o_se = take(n_out * sizeof(double));
-    const size_t o_ctl = take(kCtlBytes);   // queue head, error flags, exponential-branch steps
+    const size_t o_acc_sum = take((size_t)n_out * kLimbs * sizeof(unsigned long long));
+    db.clear_bytes = o_ctl + kCtlBytes - o_acc;
+    db.out_bytes = o_se + n_out * sizeof(double) - o_ctl;
+    db.out_bytes_acc = o_acc_sum + (size_t)n_out * kLimbs * sizeof(unsigned long long) - o_ctl;
     CvPlan cvp;                              // the control variate's analytic part (host vectors until the sync)
     if (!bp.cv.empty()) cv_plan(bp, cvp);
     const size_t o_cv = take(cvp.bytes);
@@ -182,12 +187,8 @@ hexo_status batch_upload(hexo_ctx *ctx, BatchPlan &&plan, bool f32, DeviceBatch 
         if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc batch");
         db.dcap = db.bytes;
     }
-    // pinned host mirror of outputs: price, se, acc, ctl
-    size_t hoff = 0;
-    const size_t h_price = hoff; hoff = align_up(hoff + n_out * sizeof(double), 64);
-    const size_t h_se = hoff; hoff = align_up(hoff + n_out * sizeof(double), 64);
-    const size_t h_acc = hoff; hoff = align_up(hoff + (size_t)n_out * kLimbs * sizeof(unsigned long long), 64);
-    const size_t h_ctl = hoff; hoff = align_up(hoff + kCtlBytes, 64);
+    // pinned host mirror of the control block and the outputs, laid out as on the device
+    const size_t hoff = db.out_bytes_acc;
     if (db.hmem == nullptr || db.hcap < hoff) {
         db.hmem = nullptr;
         db.own_h = true;
@@ -197,10 +198,10 @@ hexo_status batch_upload(hexo_ctx *ctx, BatchPlan &&plan, bool f32, DeviceBatch 
     }
     char *d = static_cast<char *>(db.dmem);
     char *h = static_cast<char *>(db.hmem);
-    db.h_price = reinterpret_cast<double *>(h + h_price);
-    db.h_se = reinterpret_cast<double *>(h + h_se);
-    db.h_acc = reinterpret_cast<unsigned long long *>(h + h_acc);
-    db.h_ctl = reinterpret_cast<uint32_t *>(h + h_ctl);
+    db.h_ctl = reinterpret_cast<uint32_t *>(h);
+    db.h_price = reinterpret_cast<double *>(h + (o_price - o_ctl));
+    db.h_se = reinterpret_cast<double *>(h + (o_se - o_ctl));
+    db.h_acc = reinterpret_cast<unsigned long long *>(h + (o_acc_sum - o_ctl));
 
     KernelArgs &a = db.args;
     std::memset(&a, 0, sizeof(a));
@@ -263,10 +264,7 @@ hexo_status batch_upload(hexo_ctx *ctx, BatchPlan &&plan, bool f32, DeviceBatch 
 cudaError_t batch_enqueue(DeviceBatch &db, cudaStream_t st, bool copy_acc) {
     const uint32_t n_out = db.plan.n_out;
     cudaError_t e;
-    if ((e = cudaMemsetAsync(db.args.acc, 0, (size_t)db.n_slots * n_out * kLimbs * sizeof(unsigned long long), st)) !=
-        cudaSuccess)
-        return e;
-    if ((e = cudaMemsetAsync(db.args.queue, 0, kCtlBytes, st)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(db.args.acc, 0, db.clear_bytes, st)) != cudaSuccess) return e;
     // inside a stream capture the timing events become event-record nodes of the graph
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if ((e = cudaStreamIsCapturing(st, &cap)) != cudaSuccess) return e;
@@ -291,12 +289,7 @@ cudaError_t batch_enqueue(DeviceBatch &db, cudaStream_t st, bool copy_acc) {
     fa.carry = db.carry;
     fa.carry_row = db.d_carry_row;
     if ((e = launch_finalize(fa, st)) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(db.h_price, db.d_price, n_out * sizeof(double), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(db.h_se, db.d_se, n_out * sizeof(double), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
-    if (copy_acc)
-        if ((e = cudaMemcpyAsync(db.h_acc, db.d_acc_sum, (size_t)n_out * kLimbs * sizeof(unsigned long long),
-                                 cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
-    return cudaMemcpyAsync(db.h_ctl, db.args.queue, kCtlBytes, cudaMemcpyDeviceToHost, st);
+    return cudaMemcpyAsync(db.h_ctl, db.args.queue, copy_acc ? db.out_bytes_acc : db.out_bytes, cudaMemcpyDeviceToHost, st);
 }
 
 hexo_status batch_wait(DeviceBatch &db) {

@@ -39,6 +39,7 @@ struct DeviceBatch {
     unsigned long long *d_acc_sum = nullptr;   // totals of the private sum copies
     void *dmem = nullptr;
     size_t bytes = 0;
+    size_t clear_bytes = 0, out_bytes = 0, out_bytes_acc = 0;   // from the sums; from the control block, without and with the limbs
     void *hmem = nullptr;
     // Memory handed in before upload is reused when large enough (own_* false:
     // the batch does not free it); otherwise the upload allocates its own.
