@@ -301,7 +301,7 @@ struct Exp {                 // one expiry of one request
     uint64_t tw_off, h_off, v_off, w_off, o_off;  // element offsets into the work buffers
     uint32_t logN, logR;     // N = 2J in R parts (the transforms by FFT), or logN = 0: direct sums
     uint64_t y_off;          // its N results of a transform's parts
-    uint32_t stiff, pad;     // see kStiff
+    uint32_t stiff, logL;    // see kStiff; folded segments of 2^logL frequencies (price_kernel), or 0
 };
 
 // Expiries with fewer frequencies than this use the direct sums (automatic
@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(128) setup_kernel(const Exp *ex, const Item *i
     Opt o;
     o.x = E.r * E.tau + log(E.S / K);
     o.f = exp(-E.r * E.tau) * K;
-    sincos(64.0 * E.du * o.x, &o.ts, &o.tc);
+    if (!E.stiff && E.logL == 0u) sincos(64.0 * E.du * o.x, &o.ts, &o.tc);
     opts[E.o_off + n] = o;
 }
 
@@ -571,40 +571,100 @@ __global__ void __launch_bounds__(64) density_kernel(const Exp *ex, const Item *
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
         const cplx w = g[q] * c;
-        W[E.w_off + (uint64_t)q * E.J + j] = make_double2(w.re, w.im);
+        double2 *Wq = W + E.w_off + (uint64_t)q * E.J;
+        if constexpr (!kStiffForm)
+            if (E.logL) {   // full warps: J is a multiple of the block
+                const uint32_t L = 1u << E.logL, at = j & (L - 1u), seg = j >> E.logL;
+                const bool up = at >= L / 2;
+                const double a = up ? w.re : w.im, b = up ? w.im : w.re;
+                Wq[((((seg >> 5) << E.logL) + at) << 5) + (seg & 31u)] =
+                    make_double2(a + __shfl_xor_sync(0xffffffffu, b, L - 1u),    // the partner's b is of a's part
+                                 b - __shfl_xor_sync(0xffffffffu, a, L - 1u));
+                continue;
+            }
+        Wq[j] = make_double2(w.re, w.im);
     }
 }
 
-// One warp per option: Re sum_j W_q(j) disc K e^{-i u_j x}.  A lane's terms
-// are 32 j apart, so its phase turns by e^{-i 64 du x} from one to the next:
-// one complex product instead of a sincos (4 FP64 instructions instead of
-// a sincos's 45, or 15 by table), and a sincos every 16 terms, so that the products' roundings do
-// not add up beyond the sincos argument's own.  kGrad: the gradient too.
+// One warp per option: Re sum_j W_q(j) disc K e^{-i u_j x}, FP64-pipe bound.
+//
+// From kFoldMinJ frequencies a lane takes segments of L = 2^logL <= 32
+// consecutive ones and folds each about its centre: the frequencies of a pair
+// are u_c -+ b_k, b_k = (2k + 1) du, so with (x, y) the parts of W and -, + for
+// the lower and the upper one, the pair's two terms are
+//   cos(u_c x) [(x+ + x-) cos b_k x + (y+ - y-) sin b_k x]
+// + sin(u_c x) [(y+ + y-) cos b_k x - (x+ - x-) sin b_k x].
+// density_kernel stores the four sums and differences; the b_k are the same
+// for all segments, a sincos in each of L/2 lanes; and what is left is the
+// products themselves, 24 FP64 instructions a pair with the gradient (4
+// without) and a sincos and 12 (2) a segment: 1.70 -> 1.46 ms on 2,048 chains of
+// 50 strikes at J = 64 to 4096, 16.2 -> 13.3 us on a calibration's
+// eight.  At J = 256 (segments of 8) both forms count 140 instructions a lane,
+// and the fold's longer chain made the calibration's 19.8 us.
+// Fewer frequencies, where those do not pay: a lane's terms are 32 j apart, so its
+// phase turns by e^{-i 64 du x} from one to the next, one complex product
+// instead of a sincos (4 FP64 instructions instead of a sincos's 45, or 15 by
+// table), 32 a pair with the gradient, and a sincos every 16 terms, so that
+// the products' roundings do not add up beyond the sincos argument's own.
+// kGrad: the gradient too.
 constexpr uint32_t kTurns = 16;
+constexpr uint32_t kFoldMinJ = 512, kLogFold = 5;
 template <bool kGrad>
 __global__ void __launch_bounds__(128) price_kernel(const Exp *ex, const Item *items, const double2 *W,
                                                     const Opt *opts, double *price, double *grad) {
+    __shared__ double2 turns[4][1u << (kLogFold - 1)];   // a warp's (cos, sin) b_k x
     const Exp &E = ex[items[blockIdx.x].e];
     const uint32_t i = items[blockIdx.x].first + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
     if (i >= E.n_opt) return;   // warp-uniform
     const Opt o = opts[E.o_off + i];
     constexpr int kQ = kGrad ? 6 : 1;
     double acc[6] = {0, 0, 0, 0, 0, 0};
-    const uint32_t span = 32u * (E.stiff ? 1u : kTurns);
-    for (uint32_t j0 = lane; j0 < E.J; j0 += span) {
-        double s, c;     // e^{-i u x} = c - i s
-        if (E.stiff) sincos((2.0 * j0 + 1.0) * E.du * o.x, &s, &c);
-        else f64::sincos_tab((2.0 * j0 + 1.0) * E.du * o.x, &s, &c);
-        const uint32_t j1 = min(E.J, j0 + span);
-        for (uint32_t j = j0; j < j1; j += 32) {
+    if (E.logL) {
+        const uint32_t half = 1u << (E.logL - 1u);
+        double2 *b = turns[threadIdx.x >> 5];
+        if (lane < half) {
+            double s, c;
+            f64::sincos_tab((2.0 * lane + 1.0) * E.du * o.x, &s, &c);
+            b[lane] = make_double2(c, s);
+        }
+        __syncwarp();
+        for (uint32_t seg = lane; (seg << E.logL) < E.J; seg += 32u) {
+            const double2 *Ws = W + E.w_off + (((uint64_t)(seg >> 5) << E.logL) << 5) + lane;
+            double s, c, P[kQ], Q[kQ];
+            f64::sincos_tab(((double)seg * 2.0 + 1.0) * (double)(half << 1) * E.du * o.x, &s, &c);
 #pragma unroll
-            for (int q = 0; q < kQ; ++q) {
-                const double2 w = W[E.w_off + (uint64_t)q * E.J + j];
-                acc[q] = fma(w.x, c, fma(w.y, s, acc[q]));
+            for (int q = 0; q < kQ; ++q) P[q] = Q[q] = 0.0;
+#pragma unroll 2
+            for (uint32_t k = 0; k < half; ++k) {
+                const double2 t = b[k];
+#pragma unroll
+                for (int q = 0; q < kQ; ++q) {
+                    const double2 w = Ws[(uint64_t)q * E.J + ((half + k) << 5)];
+                    const double2 m = Ws[(uint64_t)q * E.J + ((half - 1u - k) << 5)];
+                    P[q] = fma(w.x, t.x, fma(w.y, t.y, P[q]));
+                    Q[q] = fma(m.x, t.x, fma(m.y, t.y, Q[q]));
+                }
             }
-            const double c1 = fma(c, o.tc, -s * o.ts);
-            s = fma(c, o.ts, s * o.tc);
-            c = c1;
+#pragma unroll
+            for (int q = 0; q < kQ; ++q) acc[q] = fma(c, P[q], fma(s, Q[q], acc[q]));
+        }
+    } else {
+        const uint32_t span = 32u * (E.stiff ? 1u : kTurns);
+        for (uint32_t j0 = lane; j0 < E.J; j0 += span) {
+            double s, c;     // e^{-i u x} = c - i s
+            if (E.stiff) sincos((2.0 * j0 + 1.0) * E.du * o.x, &s, &c);
+            else f64::sincos_tab((2.0 * j0 + 1.0) * E.du * o.x, &s, &c);
+            const uint32_t j1 = min(E.J, j0 + span);
+            for (uint32_t j = j0; j < j1; j += 32) {
+#pragma unroll
+                for (int q = 0; q < kQ; ++q) {
+                    const double2 w = W[E.w_off + (uint64_t)q * E.J + j];
+                    acc[q] = fma(w.x, c, fma(w.y, s, acc[q]));
+                }
+                const double c1 = fma(c, o.tc, -s * o.ts);
+                s = fma(c, o.ts, s * o.tc);
+                c = c1;
+            }
         }
     }
     if constexpr (kGrad) {   // lanes 0-15 take on the first three sums, 16-31 the others
@@ -780,6 +840,7 @@ hexo_status hexo_swift_price(hexo_ctx *ctx, const hexo_swift_request *reqs, uint
             e.v_off = v;
             v += (uint64_t)(sp.k2 - sp.k1 + 1);
         }
+        e.logL = e.stiff || sp.J < kFoldMinJ ? 0u : std::min(logJ - 5u, kLogFold);
         if (tw_at.off[logJ] == ~0ull) {
             tw_at.off[logJ] = tw;
             for (uint32_t n = 0; n < 4 * sp.J; n += 128) it_set.push_back({logJ, n});

@@ -51,3 +51,9 @@ def test_far_frequencies(engine, oracle):
     # u up to 2^9 pi: d tau / 2 passes 300 (phi is below e^-300 there)
     p5 = [0.04, 0.05, -0.3, 1.5, 0.9]
     check(engine, oracle, p5, 4.0, (8, 256, 16.0, -4.0, 4.0, -1000, 1000, 1024), 0)
+
+
+@pytest.mark.parametrize("J", [256, 512, 2048, 4096])   # below the folds; segments of 16 and 32, one to four rounds
+@pytest.mark.parametrize("method", [1, 2])
+def test_folded_segments(engine, oracle, J, method):
+    check(engine, oracle, P5, 0.3, (6, 64, 8.0, -3.0, 3.0, -192, 191, J), method)
