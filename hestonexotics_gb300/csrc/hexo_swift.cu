@@ -951,7 +951,13 @@ hexo_status hexo_swift_price(hexo_ctx *ctx, const hexo_swift_request *reqs, uint
                                                 (int)(sizeof(double2) << kLogMaxPart))) != cudaSuccess)
                     return cuda_fail(ctx, err, "swift shared memory");
         fft_terms_kernel<<<(unsigned)it_fft.size(), 128, smem, st>>>(dex, items(o_if), dtw, dh, dy);
-        fft_payoff_kernel<<<(unsigned)it_fft.size(), 128, smem, st>>>(dex, items(o_if), dtw, dy, dz);
+        // Where the parts fill the GPU several times over, blocks of two warps: a part of a common
+        // expiry (J = 256 to 1024: 64 to 256 points) keeps its warps busy, and at 142 registers
+        // more parts are resident: 0.41 -> 0.30 ms on 2,048 chains (fft_terms_kernel, 32
+        // registers: 0.13 -> 0.14).  Fewer parts want every warp that a part can use: half of
+        // them would leave half of an SM's FP64 units idle.
+        const unsigned width = it_fft.size() >= 4ull * ctx->sm_count ? 64u : 128u;
+        fft_payoff_kernel<<<(unsigned)it_fft.size(), width, smem, st>>>(dex, items(o_if), dtw, dy, dz);
     }
     if (!it_pay.empty()) payoff_kernel<<<(unsigned)it_pay.size(), 32, 0, st>>>(dex, items(o_ip), dtw, dh, dv);
     if (!it_den.empty())

@@ -57,3 +57,15 @@ def test_far_frequencies(engine, oracle):
 @pytest.mark.parametrize("method", [1, 2])
 def test_folded_segments(engine, oracle, J, method):
     check(engine, oracle, P5, 0.3, (6, 64, 8.0, -3.0, 3.0, -192, 191, J), method)
+
+
+def test_many_parts(engine):
+    # enough parts for the narrow FFT blocks (8 an expiry, 4 a multiprocessor): the same operations
+    # in the same order as in an expiry's call of its own, so the same bits
+    sps = [(4, 16, 4.0, -3.0, 3.0, -int(1.1 * J) - 1, int(1.7 * J) + 1, J) for J in (2, 16, 32, 64, 256, 1024, 4096)]
+    chains = [(0.5, K)] * (16 * len(sps))
+    many = engine.swift(E.Params(*P5, r=0.02), 100.0, chains, grad=True, swift_params=sps * 16, method=2)
+    for (price, grad), sp in zip(many, sps * 16):
+        (p1, g1), = engine.swift(E.Params(*P5, r=0.02), 100.0, chains[:1], grad=True, swift_params=[sp], method=2)
+        np.testing.assert_array_equal(price, p1)
+        np.testing.assert_array_equal(grad, g1)
