@@ -15,9 +15,9 @@
 // evaluated with Gauss-Legendre on [0, U] (256 nodes) and, through u = U / s,
 // on [U, inf) (128 nodes), U = 40 standard deviations of L.
 //
-// One thread per (maturity, node) runs the recursion in FP64 complex
-// arithmetic; one thread per option then sums the nodes.  Done once when a
-// batch is uploaded; the finaliser combines it with the path sums.
+// One warp or one thread per (maturity, node) runs the recursion in FP64
+// complex arithmetic; one warp per option then sums the nodes.  Done once when
+// a batch is uploaded; the finaliser combines it with the path sums.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <algorithm>
@@ -460,7 +460,7 @@ cudaError_t cv_run(const CvPlan &cp, void *region, cudaStream_t st, double **eg,
     if (e == cudaSuccess) e = up(d_nodes, cp.nodes.data(), cp.nodes.size() * sizeof(double2));
     if (e != cudaSuccess || cp.n_mats == 0) return e;
     // the recursion is bound by each SM's FP64 pipe: sets with few maturities one warp per
-    // (maturity, node) over the steps (about 1.5 times the arithmetic, over 32 lanes), the
+    // (maturity, node) over the steps (each step's map evaluated twice, over 32 lanes), the
     // rest one thread per pair, one warp per block so that the pairs spread over the SMs
     if (cp.n_warp_mats > 0) {
         const uint64_t n_thr = (uint64_t)cp.n_warp_mats * (kCvNodes + 1) * 32u;
