@@ -331,6 +331,15 @@ struct Opt {
     double x, f, ts, tc;
 };
 
+// A call's kernels follow one another within microseconds, so each may be
+// launched while the one before runs (Launches) and waits here, before it
+// touches memory, until that one has ended and its results are visible; every
+// kernel waits, so the ones before that have ended too.
+__device__ __forceinline__ void after_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // The tables of a call in one launch, n_tw + n_h + n_o blocks of 128 threads:
 // w^n = e^{i pi n / (2J)} for n < 4J, one table per distinct J (items: log2 J,
 // first n); the payoff terms h_j, one thread per j; and the options' terms,
@@ -339,6 +348,7 @@ struct Opt {
 __global__ void __launch_bounds__(128) setup_kernel(const Exp *ex, const Item *items, uint32_t n_tw, uint32_t n_h,
                                                     const TwiddleAt at, const double *strikes, double2 *tw, double2 *h,
                                                     Opt *opts) {
+    after_previous();
     const Item it = items[blockIdx.x];
     const uint32_t n = it.first + threadIdx.x;
     if (blockIdx.x < n_tw) {
@@ -426,6 +436,7 @@ __device__ __forceinline__ uint32_t bit_reverse(uint32_t i, uint32_t ln) { retur
 __global__ void __launch_bounds__(128) fft_terms_kernel(const Exp *ex, const Item *items, const double2 *tw,
                                                         const double2 *h, double2 *y) {
     extern __shared__ double2 s[];
+    after_previous();
     const Exp &E = ex[items[blockIdx.x].e];
     const uint32_t r = items[blockIdx.x].first, J = E.J, ln = E.logN - E.logR, n = 1u << ln;
     for (uint32_t l = threadIdx.x; l < n; l += blockDim.x) {
@@ -492,6 +503,7 @@ __device__ __forceinline__ void load_payoffs(const Exp &E, uint32_t r, double2 *
 __global__ void __launch_bounds__(128) fft_payoff_kernel(const Exp *ex, const Item *items, const double2 *tw,
                                                          const double2 *y, double2 *z) {
     extern __shared__ double2 s[];
+    after_previous();
     const Exp &E = ex[items[blockIdx.x].e];
     const uint32_t r = items[blockIdx.x].first, ln = E.logN - E.logR, n = 1u << ln;
     const double2 *T = tw + E.tw_off, *Y = y + E.y_off;
@@ -525,6 +537,7 @@ __device__ __forceinline__ double2 fft_output(const double2 *z, uint32_t j, uint
 
 // V_k by the direct sum, one lane per k
 __global__ void payoff_kernel(const Exp *ex, const Item *items, const double2 *tw, const double2 *h, double *V) {
+    after_previous();
     const Exp &E = ex[items[blockIdx.x].e];
     const int32_t k = E.k1 + (int32_t)(items[blockIdx.x].first + threadIdx.x);
     if (k > E.k2) return;
@@ -547,6 +560,7 @@ __global__ void payoff_kernel(const Exp *ex, const Item *items, const double2 *t
 template <bool kStiffForm>
 __global__ void __launch_bounds__(64) density_kernel(const Exp *ex, const Item *items, const double2 *tw,
                                                      const double *V, double2 *W, const double2 *z) {
+    if constexpr (!kStiffForm) after_previous();   // the stiff form is launched the ordinary way
     const Exp E = ex[items[blockIdx.x].e];   // a copy: the stiff form's contractions depend on it
     const uint32_t j = items[blockIdx.x].first + threadIdx.x;
     if (j >= E.J) return;
@@ -624,6 +638,7 @@ template <bool kGrad>
 __global__ void __launch_bounds__(128) price_kernel(const Exp *ex, const Item *items, const double2 *W,
                                                     const Opt *opts, double *price, double *grad) {
     __shared__ double2 turns[4][1u << (kLogFold - 1)];   // a warp's (cos, sin) b_k x
+    after_previous();
     const Exp &E = ex[items[blockIdx.x].e];
     const uint32_t i = items[blockIdx.x].first + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
     if (i >= E.n_opt) return;   // warp-uniform
@@ -709,6 +724,33 @@ using namespace hexo;
 using namespace hexo::swift;
 
 namespace {
+
+// A call's launches.  A kernel may begin while the one before it still runs
+// (it starts with after_previous()), where the blocks of both find an SM each:
+// a calibration's eight expiries 275 -> 260 us a step, one chain of 50 strikes
+// at J = 512 134 -> 108 us.  Larger grids are launched when the one before has
+// ended: early blocks share the SMs that it left free and run unevenly (one
+// chain of 2,000 strikes at J = 16,384 0.50 -> 0.73 ms).
+struct Launches {
+    cudaStream_t st;
+    uint64_t sm_count;
+    uint64_t last;   // blocks of the kernel before
+    template <class... P, class... A>
+    void run(size_t grid, unsigned block, size_t smem, void (*k)(P...), A... a) {   // errors: cudaGetLastError
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t c{};
+        c.gridDim = dim3((unsigned)grid);
+        c.blockDim = dim3(block);
+        c.dynamicSmemBytes = smem;
+        c.stream = st;
+        c.attrs = &at;
+        c.numAttrs = last + grid <= sm_count ? 1u : 0u;
+        last = grid;
+        cudaLaunchKernelEx(&c, k, static_cast<P>(a)...);
+    }
+};
 
 hexo_status params_dynamic(const HP &p, double tau, double r, double S, double K_min, double K_max, double prec,
                            hexo_swift_params &out) {
@@ -941,6 +983,7 @@ hexo_status hexo_swift_price(hexo_ctx *ctx, const hexo_swift_request *reqs, uint
             *dz = reinterpret_cast<double2 *>(d + o_z);
     double *dp = reinterpret_cast<double *>(d + o_p), *dg = any_grad ? reinterpret_cast<double *>(d + o_g) : nullptr;
     Opt *dopt = reinterpret_cast<Opt *>(d + o_o);
+    Launches go{st, ctx->sm_count, it_set.size()};
     setup_kernel<<<(unsigned)it_set.size(), 128, 0, st>>>(dex, items(o_is), n_tw, n_h, tw_at,
                                                           reinterpret_cast<const double *>(d + o_k), dtw, dh, dopt);
     if (!it_fft.empty()) {
@@ -950,22 +993,24 @@ hexo_status hexo_swift_price(hexo_ctx *ctx, const hexo_swift_request *reqs, uint
                 if ((err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 (int)(sizeof(double2) << kLogMaxPart))) != cudaSuccess)
                     return cuda_fail(ctx, err, "swift shared memory");
-        fft_terms_kernel<<<(unsigned)it_fft.size(), 128, smem, st>>>(dex, items(o_if), dtw, dh, dy);
+        go.run(it_fft.size(), 128, smem, fft_terms_kernel, dex, items(o_if), dtw, dh, dy);
         // Where the parts fill the GPU several times over, blocks of two warps: a part of a common
         // expiry (J = 256 to 1024: 64 to 256 points) keeps its warps busy, and at 142 registers
         // more parts are resident: 0.41 -> 0.30 ms on 2,048 chains (fft_terms_kernel, 32
         // registers: 0.13 -> 0.14).  Fewer parts want every warp that a part can use: half of
         // them would leave half of an SM's FP64 units idle.
         const unsigned width = it_fft.size() >= 4ull * ctx->sm_count ? 64u : 128u;
-        fft_payoff_kernel<<<(unsigned)it_fft.size(), width, smem, st>>>(dex, items(o_if), dtw, dy, dz);
+        go.run(it_fft.size(), width, smem, fft_payoff_kernel, dex, items(o_if), dtw, dy, dz);
     }
-    if (!it_pay.empty()) payoff_kernel<<<(unsigned)it_pay.size(), 32, 0, st>>>(dex, items(o_ip), dtw, dh, dv);
+    if (!it_pay.empty()) go.run(it_pay.size(), 32, 0, payoff_kernel, dex, items(o_ip), dtw, dh, dv);
     if (!it_den.empty())
-        density_kernel<false><<<(unsigned)it_den.size(), 64, 0, st>>>(dex, items(o_id), dtw, dv, dw, dz);
-    if (!it_stiff.empty())
+        go.run(it_den.size(), 64, 0, density_kernel<false>, dex, items(o_id), dtw, dv, dw, dz);
+    if (!it_stiff.empty()) {
+        go.last = it_stiff.size();
         density_kernel<true><<<(unsigned)it_stiff.size(), 64, 0, st>>>(dex, items(o_it), dtw, dv, dw, dz);
-    if (any_grad) price_kernel<true><<<(unsigned)it_pri.size(), 128, 0, st>>>(dex, items(o_ir), dw, dopt, dp, dg);
-    else price_kernel<false><<<(unsigned)it_pri.size(), 128, 0, st>>>(dex, items(o_ir), dw, dopt, dp, dg);
+    }
+    if (any_grad) go.run(it_pri.size(), 128, 0, price_kernel<true>, dex, items(o_ir), dw, dopt, dp, dg);
+    else go.run(it_pri.size(), 128, 0, price_kernel<false>, dex, items(o_ir), dw, dopt, dp, dg);
     if ((err = cudaGetLastError()) != cudaSuccess) return cuda_fail(ctx, err, "swift kernels");
     if ((err = cudaMemcpyAsync(host, dp, down_bytes, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
         (err = cudaStreamSynchronize(st)) != cudaSuccess)
