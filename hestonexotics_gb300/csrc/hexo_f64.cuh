@@ -58,8 +58,8 @@ __device__ __forceinline__ double join(ds::F2 x) {
 
 // x - a b for doubles with |x - a b| < 2^-33 2^(ea+eb) (ea, eb the exponents
 // of a and b): words 1 and 2 of the significands' product taken from x's,
-// cut at 2^-64 of 2^(ea+eb).
-__device__ __forceinline__ float remainder_mul(double x, double a, double b) {
+// cut at 2^-64 of 2^(ea+eb) (the unit of the integer forms).
+__device__ __forceinline__ int32_t remainder_mul_units(double x, double a, double b) {
     const uint32_t al = lo32(a), bl = lo32(b), ah = hi32(a), bh = hi32(b), xl = lo32(x), xh = hi32(x);
     const uint32_t am = (ah & 0x000fffffu) | 0x00100000u, bm = (bh & 0x000fffffu) | 0x00100000u;
     uint64_t p = (uint64_t)al * bm + __umulhi(al, bl);
@@ -67,20 +67,25 @@ __device__ __forceinline__ float remainder_mul(double x, double a, double b) {
     p += (uint64_t)(am * bm) << 32;
     const uint32_t s = 20u + 1023u + (xh >> 20) - (ah >> 20) - (bh >> 20);   // 19 to 22
     const uint64_t d = (((uint64_t)__funnelshift_l(xl, xh, s) << 32) | (uint64_t)(uint32_t)(xl << s)) - p;
-    const int32_t r = (int32_t)__funnelshift_r((uint32_t)d, (uint32_t)(d >> 32), 8);
-    return __fmul_rn(__fmul_rn(__fmul_rn(__int2float_rn(r), 0x1p-64f), pow2_of(a)), pow2_of(b));
+    return (int32_t)__funnelshift_r((uint32_t)d, (uint32_t)(d >> 32), 8);
+}
+__device__ __forceinline__ float remainder_mul(double x, double a, double b) {
+    const float r = __int2float_rn(remainder_mul_units(x, a, b));
+    return __fmul_rn(__fmul_rn(__fmul_rn(r, 0x1p-64f), pow2_of(a)), pow2_of(b));
 }
 // x - q^2
-__device__ __forceinline__ float remainder_sqr(double x, double q) {
+__device__ __forceinline__ int32_t remainder_sqr_units(double x, double q) {
     const uint32_t ql = lo32(q), qh = hi32(q), xl = lo32(x), xh = hi32(x);
     const uint32_t qm = (qh & 0x000fffffu) | 0x00100000u;
     uint64_t p = (uint64_t)ql * (qm + qm) + __umulhi(ql, ql);
     p += (uint64_t)(qm * qm) << 32;
     const uint32_t s = 20u + 1023u + (xh >> 20) - 2u * (qh >> 20);
     const uint64_t d = (((uint64_t)__funnelshift_l(xl, xh, s) << 32) | (uint64_t)(uint32_t)(xl << s)) - p;
-    const int32_t r = (int32_t)__funnelshift_r((uint32_t)d, (uint32_t)(d >> 32), 8);
-    const float e = pow2_of(q);
-    return __fmul_rn(__fmul_rn(__fmul_rn(__int2float_rn(r), 0x1p-64f), e), e);
+    return (int32_t)__funnelshift_r((uint32_t)d, (uint32_t)(d >> 32), 8);
+}
+__device__ __forceinline__ float remainder_sqr(double x, double q) {
+    const float r = __int2float_rn(remainder_sqr_units(x, q)), e = pow2_of(q);
+    return __fmul_rn(__fmul_rn(__fmul_rn(r, 0x1p-64f), e), e);
 }
 
 // ------------------------------------------------------------------ tables
@@ -278,20 +283,27 @@ __device__ __forceinline__ uint64_t neg_log_fixed(uint64_t P, int k, float d) {
     return (int64_t)l < 0 ? 0ull - l : 0ull;
 }
 
-// sqrt(x), within 0.51 ulp (x below 2^-120, 0 included, gives a root below
-// 2^-59): the remainder's correction is added to the bits of the joined root
-// in units of its last place.  No FP64 instruction (the library's root takes
-// the time of 7).
+// Whether a joined value lies within 2^-20 of a power of two.  There the unit
+// of its last place need not be the seed's, and a correction can carry it over
+// into the next binade, where the same bits count twice or half as much: the
+// root and the reciprocal below take the plain operation for these.
+__device__ __forceinline__ bool near_binade(double y) { return (hi32(y) << 12) + 0x1000u <= 0x1000u; }
+
+// sqrt(x), within 0.51 ulp from 2^-113 on: the remainder's correction is added
+// to the bits of the joined root in units of its last place.  Below, the seed's
+// float remainder runs out of bits (relative error 2^-31 at 2^-119), and x
+// below 2^-120, 0 included, gives a root of about 2^-60.  No FP64 instruction
+// but for one value in 2^19 (the library's root takes the time of 7).
 __device__ __forceinline__ double root(double x) {
-    if ((int)hi32(x) >= 0x46300000) return __dsqrt_rn(x);   // x >= 2^100, infinite or NaN
-    const uint32_t h = (uint32_t)max((int)hi32(x), 0x38700000);
+    const uint32_t h = (uint32_t)max((int)hi32(x), 0x38700800);   // not a power of two: 0 is common
     const double xc = from_words(h, lo32(x));
     const ds::F2 xs = split(xc);
     const float hr = __fmul_rn(0.5f, ds::rsqrt_approx(xs.h));
     const float s0 = __fmul_rn(__fadd_rn(xs.h, xs.h), hr);
     const double S = join(ds::fast_two_sum(s0, __fmul_rn(__fadd_rn(__fmaf_rn(-s0, s0, xs.h), xs.l), hr)));
-    const float unit = __uint_as_float(0x7f000000u + (52u << 23) - (__float_as_uint(s0) & 0x7f800000u));
-    const int32_t k = __float2int_rn(__fmul_rn(__fmul_rn(remainder_sqr(xc, S), hr), unit));
+    if ((int)hi32(x) >= 0x46300000 || near_binade(S)) return __dsqrt_rn(x);   // x >= 2^100, infinite or NaN
+    const float u = __fmul_rn(__fmul_rn(pow2_of(S), hr), 0x1p-12f);           // 2^-64 of the remainder's unit, in ulp of S
+    const int32_t k = __float2int_rn(__fmul_rn(__int2float_rn(remainder_sqr_units(xc, S)), u));
     return __longlong_as_double(__double_as_longlong(S) + (long long)k);
 }
 
@@ -308,14 +320,15 @@ __device__ __forceinline__ double mul_float(float z, double k) {
     return __longlong_as_double((long long)((((uint64_t)(zb & 0x80000000u)) << 32) + ((uint64_t)e << 52) + ((P + 1024ull) >> 11)));
 }
 
-// 1 / x within 0.51 ulp, 2^-60 < x < 2^60, like root without an FP64 instruction.
+// 1 / x within 0.51 ulp, 2^-60 <= x < 2^60, like root without an FP64 instruction.
 __device__ __forceinline__ double recip(double x) {
     const ds::F2 xs = split(x);
     const float r = ds::rcp_approx(xs.h);
     const ds::F2 y = ds::fast_two_sum(r, __fmul_rn(__fmaf_rn(-r, xs.l, __fmaf_rn(-r, xs.h, 1.0f)), r));
     const double Y = join(y);
-    const float unit = __uint_as_float(0x7f000000u + (52u << 23) - (__float_as_uint(y.h) & 0x7f800000u));
-    const int32_t k = __float2int_rn(__fmul_rn(__fmul_rn(remainder_mul(1.0, x, Y), r), unit));
+    if (near_binade(Y)) return 1.0 / x;
+    const float u = __fmul_rn(__fmul_rn(pow2_of(x), r), 0x1p-12f);
+    const int32_t k = __float2int_rn(__fmul_rn(__int2float_rn(remainder_mul_units(1.0, x, Y)), u));
     return __longlong_as_double(__double_as_longlong(Y) + (long long)k);
 }
 

@@ -1,0 +1,62 @@
+"""The FP64 form's own roots, reciprocals and exponential, on the host (CPU).
+
+csrc/hexo_f64.cuh uses only integer and individually rounded operations, so it
+compiles for the host (tests/device_math/host_device.h) and gives the device's
+results there but for the two approximate instructions, whose results are the
+correctly rounded ones moved by -1, 0 or 1 unit of the last place: a function
+has to keep its bound with each of those seeds.
+"""
+import ctypes as C
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT
+
+FN = {"recip": 0, "root": 1, "exp": 2}
+
+
+@pytest.fixture(scope="module")
+def f64(tmp_path_factory):
+    if shutil.which("g++") is None:
+        pytest.skip("no host compiler")
+    so = tmp_path_factory.mktemp("device_math") / "f64_host.so"
+    r = subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-fconstexpr-ops-limit=200000000", "-shared",
+                        "-fPIC", "-I", str(ROOT / "hestonexotics_gb300" / "csrc"),
+                        str(ROOT / "tests" / "device_math" / "f64_host.cpp"), "-o", str(so)],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-4000:]
+    lib = C.CDLL(str(so))
+    lib.f64_worst_ulp.restype = C.c_double
+
+    def worst(fn, seed, x):
+        x = np.ascontiguousarray(x, dtype=np.float64)
+        at = C.c_double()
+        w = lib.f64_worst_ulp(FN[fn], seed, C.c_uint64(len(x)), x.ctypes.data_as(C.c_void_p), C.byref(at))
+        return w, at.value.hex()
+    return worst
+
+
+def neighbours(e_lo, e_hi, rng):
+    """Powers of two and the doubles around them: the nearest 300 either way, and more up to 2^-20 away."""
+    k = np.concatenate([np.arange(-300, 301), (2.0 ** rng.uniform(0, 32, 400)).astype(np.int64),
+                        -(2.0 ** rng.uniform(0, 32, 400)).astype(np.int64)])
+    one = np.array([1.0]).view(np.int64) + k
+    return np.concatenate([np.ldexp(one.view(np.float64), e) for e in range(e_lo, e_hi)])
+
+
+# 0.51 units, the functions' stated bound: half a unit of the rounding and what the correction's float product adds
+@pytest.mark.parametrize("seed", [-1, 0, 1])
+@pytest.mark.parametrize("fn", ["recip", "root"])
+def test_recip_and_root_next_to_powers_of_two(f64, fn, seed):
+    w, at = f64(fn, seed, neighbours(-58, 59, np.random.default_rng(1)))
+    assert w <= 0.51, f"{w} units at {at}"
+
+
+@pytest.mark.parametrize("seed", [-1, 0, 1])
+@pytest.mark.parametrize("fn,lo,hi", [("recip", -59.9, 59.9), ("root", -112.9, 99.9)])
+def test_recip_and_root_over_their_ranges(f64, fn, lo, hi, seed):
+    w, at = f64(fn, seed, 2.0 ** np.random.default_rng(2).uniform(lo, hi, 200000))
+    assert w <= 0.51, f"{w} units at {at}"
