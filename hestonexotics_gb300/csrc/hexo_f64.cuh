@@ -217,8 +217,9 @@ __device__ __forceinline__ uint64_t sqr_hi(uint64_t r) {
     return (uint64_t)hi(r) * hi(r) + 2ull * __umulhi(hi(r), lo(r));
 }
 
-// exp(x) in integer arithmetic, within 0.6 ulp: x in units of 2^-54 is n
-// ln2/256 + r, 0 <= r < ln2/256 (1 + 2^-11), r in units of 2^-71, and the
+// exp(x) in integer arithmetic, within 0.57 ulp for |x| < 32 and 0.63 up to 512
+// (ln2/256 is kept to 2^-71): x in units of 2^-54 is n ln2/256 + r, 0 <= r <
+// ln2/256 (1 + 2^-11), r in units of 2^-71 with what x has below 2^-54, and the
 // result 2^(n/256) (1 + r + r^2/2 + r^3 (1/6 + r/24 + r^2/120)) in units of
 // 2^-62.  No FP64 instruction (the library's exp takes the time of 18).
 __device__ __forceinline__ double exp_tab(double x, const ExpTab *tab) {
@@ -226,11 +227,16 @@ __device__ __forceinline__ double exp_tab(double x, const ExpTab *tab) {
     if (a >= 0x40800000u) return exp(x);   // |x| >= 512, infinite or NaN
     const uint64_t M = ((uint64_t)((a << 10 & 0x3fffffffu) | 0x40000000u) << 32 | (uint64_t)(lo32(x) >> 22) << 32) |
                        (uint64_t)(lo32(x) << 10);
-    uint64_t F = M >> min(1031u - (a >> 20), 63u);
-    if ((int32_t)xh < 0) F = 0ull - F;
+    const uint32_t sh = 1031u - (a >> 20);
+    uint64_t F = M >> min(sh, 63u), R = F << 17;                     // units of 2^-54, 2^-71
+    if (sh - 11u < 53u) R |= ((M << 1) << (63u - sh)) >> 47;         // |x| < 1/4: bits below 2^-54
+    if ((int32_t)xh < 0) {
+        F = 0ull - F;
+        R = 0ull - R;
+    }
     const int32_t n = __mulhi((int32_t)hi(F) - 2, (int32_t)(kExpTab / kLn2.h * 0x1p22)) >> 12;
     constexpr uint64_t L71 = (uint64_t)(kLn2.h / kExpTab * 0x1p71) + (uint64_t)(int64_t)(kLn2.l / kExpTab * 0x1p71 + 0.5);
-    const uint64_t r = (F << 17) - (uint64_t)(int64_t)n * L71;
+    const uint64_t r = R - (uint64_t)(int64_t)n * L71;
     const uint32_t rh = hi(r);
     const uint32_t p = 2863311531u + __umulhi(rh, 5592405u + __umulhi(rh, 8738u));   // 1/6 + r/24 + r^2/120, 2^-34
     const uint32_t q = __umulhi(rh << 1, p) << 1;                                    // r p, 2^-43

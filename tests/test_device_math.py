@@ -60,3 +60,21 @@ def test_recip_and_root_next_to_powers_of_two(f64, fn, seed):
 def test_recip_and_root_over_their_ranges(f64, fn, lo, hi, seed):
     w, at = f64(fn, seed, 2.0 ** np.random.default_rng(2).uniform(lo, hi, 200000))
     assert w <= 0.51, f"{w} units at {at}"
+
+
+# half a unit of the rounding, 0.07 of the polynomial's 32-bit terms and the table's 2^-62, and, where |x| is
+# large, n = 256 |x| / ln2 times what ln2/256 is off in units of 2^-71 (0.06 there)
+@pytest.mark.parametrize("sign", [-1.0, 1.0])
+@pytest.mark.parametrize("lo,hi,bound", [(-70, -20, 0.57), (-20, -8, 0.57), (-8, -2, 0.57), (-2, 5, 0.57), (5, 9, 0.63)])
+def test_exp_over_its_range(f64, sign, lo, hi, bound):
+    w, at = f64("exp", 0, sign * 2.0 ** np.random.default_rng(3).uniform(lo, hi, 200000))
+    assert w <= bound, f"{w} units at {at}"
+
+
+def test_exp_around_its_table(f64):
+    # results around every table entry and around powers of two, arguments of either sign and zero
+    n = np.arange(-5120, 5121)[:, None] * (np.log(2.0) / 256)
+    x = np.concatenate([(n + np.random.default_rng(4).uniform(-1, 1, (1, 40)) * 2.0 ** -np.arange(10, 50)).ravel(),
+                        [0.0, -0.0, 5e-324, -5e-324, 2.0 ** -54, -(2.0 ** -54), 511.9999, -511.9999]])
+    w, at = f64("exp", 0, x)
+    assert w <= 0.57, f"{w} units at {at}"
