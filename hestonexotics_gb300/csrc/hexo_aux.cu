@@ -36,8 +36,19 @@ cudaError_t paths_smem_limit(const void *fn, int dev) {
 // the control variate, against 5.4, 8.5 and 15.4 us here; a block per 32
 // options with the FP64 arithmetic a lane per option took 5.4, 12.6 and 25 us.
 static_assert(kSumSlots <= 16 && kLimbs == 6, "a warp sums 16 copies, half of the limbs in each half");
+// The option of a thread and the blocks for n options, for any n that 32 bits
+// hold (a thread's index in the grid is 32 times an option's, and would wrap
+// from 2^27 options on).
+constexpr uint32_t kFinalWarps = 4;
+__host__ __device__ constexpr uint32_t final_option(uint32_t block, uint32_t thread) {
+    return block * kFinalWarps + (thread >> 5);
+}
+constexpr uint32_t final_blocks(uint32_t n) { return n / kFinalWarps + (n % kFinalWarps != 0u ? 1u : 0u); }
+static_assert(final_option(final_blocks(0xffffffffu) - 1u, 31u + 2u * 32u) == 0xfffffffeu, "the last option's warp");
+static_assert(final_option(1u << 25, 0u) == 1u << 27, "past 2^27 options");
+static_assert(final_blocks(0xffffffffu) == 1u << 30 && final_blocks(1u) == 1u && final_blocks(4u) == 1u, "blocks");
 __global__ void finalize_kernel(const FinalizeArgs f) {
-    const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    const uint32_t i = final_option(blockIdx.x, threadIdx.x), lane = threadIdx.x & 31u;
     if (i >= f.n) return;   // warp-uniform
     auto total = [&](uint32_t o, uint64_t (&l)[kLimbs]) {
         const uint32_t s = lane & 15u, half = (lane >> 4) * 3u;
@@ -88,7 +99,7 @@ __global__ void finalize_kernel(const FinalizeArgs f) {
 
 cudaError_t launch_finalize(const FinalizeArgs &f, cudaStream_t st) {
     if (f.n == 0) return cudaSuccess;
-    finalize_kernel<<<(f.n + 3) / 4, 128, 0, st>>>(f);
+    finalize_kernel<<<final_blocks(f.n), kFinalWarps * 32u, 0, st>>>(f);
     return cudaGetLastError();
 }
 
