@@ -409,10 +409,15 @@ hexo_status hexo_ctx_create(hexo_ctx **out, const hexo_ctx_opts *opts) {
         delete ctx;
         return e == cudaErrorMemoryAllocation ? HEXO_ERR_NOMEM : HEXO_ERR_CUDA;
     }
-    if (cudaMallocHost(&ctx->pinned_keep, 64) != cudaSuccess) {   // only a matter of speed
+    // only a matter of speed; relaxed, so that it is no business of a capture that the process may have
+    // under way (in global mode an allocation by any thread would invalidate it)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    const bool swapped = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
+    if (!swapped || cudaMallocHost(&ctx->pinned_keep, 64) != cudaSuccess) {
         (void)cudaGetLastError();
         ctx->pinned_keep = nullptr;
     }
+    if (swapped) cudaThreadExchangeStreamCaptureMode(&mode);
     tune_load(ctx);
     *out = ctx;
     return HEXO_OK;
