@@ -402,7 +402,8 @@ class Engine:
         """requests: [(Params, S, [(tau, strikes), ...]), ...], priced in one call."""
         # one array each for all strikes, prices and gradients, and one of chain records (a record,
         # three arrays and four casts per chain took ten microseconds each, more than its pricing)
-        Ks = [np.ascontiguousarray(K, dtype=np.float64) for _, _, chains in requests for _, K in chains]
+        flat = [(float(tau), np.ascontiguousarray(K, dtype=np.float64)) for _, _, chains in requests for tau, K in chains]
+        Ks = [K for _, K in flat]
         ns = np.array([len(K) for K in Ks], dtype=np.int64)
         ends = np.cumsum(ns)
         total = int(ends[-1]) if len(ns) else 0
@@ -412,11 +413,12 @@ class Engine:
         at = (ends - ns).astype(np.uint64)
         arr = np.zeros(max(1, len(Ks)), dtype=_CHAIN_DTYPE)
         rec = arr[:len(Ks)]
-        rec["tau"] = [float(tau) for _, _, chains in requests for tau, _ in chains]
+        rec["tau"] = [tau for tau, _ in flat]
         rec["strikes"] = np.uint64(strikes.ctypes.data) + 8 * at
         rec["n"] = ns
-        rec["method"] = int(method)
-        rec["trunc_precision"] = trunc_precision
+        # converted as ctypes fields: numpy would refuse a method below 0 and take None, text or arrays for a number
+        rec["method"] = C.c_uint32(int(method)).value
+        rec["trunc_precision"] = C.c_double(trunc_precision).value
         rec["price_out"] = np.uint64(price.ctypes.data) + 8 * at
         if grad:
             rec["grad_out"] = np.uint64(g.ctypes.data) + 40 * at
@@ -440,12 +442,12 @@ class Engine:
         self._check(self._lib.hexo_swift_price(self._ctx, reqs, len(requests)))
         cuts = [0, *ends.tolist()]
         if grad:
-            flat = [(price[i:j], g[i:j]) for i, j in zip(cuts, cuts[1:])]
+            parts = [(price[i:j], g[i:j]) for i, j in zip(cuts, cuts[1:])]
         else:
-            flat = [price[i:j] for i, j in zip(cuts, cuts[1:])]
+            parts = [price[i:j] for i, j in zip(cuts, cuts[1:])]
         outs, first = [], 0
         for _, _, chains in requests:
-            outs.append(flat[first:first + len(chains)])
+            outs.append(parts[first:first + len(chains)])
             first += len(chains)
         return outs
 
