@@ -586,7 +586,7 @@ hexo_status hexo_batch_info_get(hexo_batch *b, hexo_batch_info *info) {
     info->grid = b->db.grid;
     info->device_bytes = b->db.bytes;
     info->h2d_bytes = b->db.h2d_bytes;
-    info->d2h_bytes = (uint64_t)bp.n_out * 2 * sizeof(double) + kCtlBytes;
+    info->d2h_bytes = b->partial ? b->db.out_bytes_acc : b->db.out_bytes;
     float ms = 0.0f;
     info->last_kernel_ms = cudaEventElapsedTime(&ms, b->db.ev_k0, b->db.ev_k1) == cudaSuccess ? (double)ms : -1.0;
     uint64_t exp_steps = 0;   // counted by the kernels; every other executed step took the quadratic branch

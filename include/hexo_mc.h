@@ -207,7 +207,8 @@ typedef struct hexo_batch_info {
     uint32_t n_tiles, n_sets, n_options, block, paths_per_thread, unroll, grid;
     uint64_t device_bytes;        /* device memory the batch holds */
     uint64_t h2d_bytes;           /* bytes uploaded when the batch is planned (descriptors) */
-    uint64_t d2h_bytes;           /* bytes copied back per run (prices, standard errors, status) */
+    uint64_t d2h_bytes;           /* bytes copied back per run, in one copy (status, prices, standard errors,
+                                     each from a 256-byte boundary on) */
     double last_kernel_ms;        /* path-kernel time of the last collected run (CUDA events) */
     uint64_t quad_steps;          /* of the last collected run: QE steps that took the quadratic branch
                                      (HSimulation.tpp:63-68); quad_steps / executed_path_steps is the
