@@ -19,7 +19,7 @@ FN = {"recip": 0, "root": 1, "exp": 2}
 
 
 @pytest.fixture(scope="module")
-def f64(tmp_path_factory):
+def lib(tmp_path_factory):
     if shutil.which("g++") is None:
         pytest.skip("no host compiler")
     so = tmp_path_factory.mktemp("device_math") / "f64_host.so"
@@ -29,8 +29,12 @@ def f64(tmp_path_factory):
                        capture_output=True, text=True)
     assert r.returncode == 0, r.stderr[-4000:]
     lib = C.CDLL(str(so))
-    lib.f64_worst_ulp.restype = C.c_double
+    lib.f64_worst_ulp.restype = lib.f64_worst_variance.restype = C.c_double
+    return lib
 
+
+@pytest.fixture(scope="module")
+def f64(lib):
     def worst(fn, seed, x):
         x = np.ascontiguousarray(x, dtype=np.float64)
         at = C.c_double()
@@ -78,3 +82,34 @@ def test_exp_around_its_table(f64):
                         [0.0, -0.0, 5e-324, -5e-324, 2.0 ** -54, -(2.0 ** -54), 511.9999, -511.9999]])
     w, at = f64("exp", 0, x)
     assert w <= 0.57, f"{w} units at {at}"
+
+
+@pytest.fixture(scope="module")
+def variance(lib):
+    def worst(seed, m, s2, rng):
+        n = len(m)
+        m, s2 = np.ascontiguousarray(m), np.ascontiguousarray(s2)
+        z = rng.standard_normal(n).astype(np.float32)
+        # uniforms all over, near 1 and next to where x = Y (1 - U) crosses 1 (the branch's zero)
+        Y = 0.5 + 0.5 * s2 / (m * m)
+        x = np.where(rng.random(n) < 0.5, rng.random(n), np.exp(-2.0 ** rng.uniform(-30, 3, n))) / np.maximum(Y, 1.0)
+        uw = (np.uint64(0) - np.clip(x * 2.0 ** 64, 1, 2.0 ** 64 * (1 - 2.0 ** -53)).astype(np.uint64))
+        near, at = np.zeros(n, dtype=np.uint8), C.c_uint64()
+        p = lambda a: a.ctypes.data_as(C.c_void_p)
+        w = lib.f64_worst_variance(seed, C.c_uint64(n), p(m), p(s2), p(z), p(uw), p(near), C.byref(at))
+        i = at.value
+        return w, near.astype(bool), f"m {m[i].hex()} s2 {s2[i].hex()} z {z[i]} uw {uw[i]:#x} near {near[i]}"
+    return worst
+
+
+# Where the step takes its own functions the error stays within 5 units of 2^-53 of the terms' size: the quadratic
+# branch rounds w and w^2 and takes two roots within half a unit each, the exponential one cuts six products and
+# sums at 2^-55 or finer and rounds Y and the result.  All of m's and s^2's range, in ratios s^2/m^2 from 2^-38 up.
+@pytest.mark.parametrize("seed", [-1, 0, 1])
+@pytest.mark.parametrize("lo,hi", [(-38, -20), (-20, -2), (-2, 3), (3, 20), (20, 60), (60, 118)])
+def test_next_variance_over_its_ranges(variance, lo, hi, seed):
+    rng = np.random.default_rng(5)
+    lm, lr = rng.uniform(-30, 30, 120000), rng.uniform(lo, hi, 120000)
+    ok = np.abs(lr + 2 * lm) < 60
+    w, near, at = variance(seed, 2.0 ** lm[ok], 2.0 ** (lr + 2 * lm)[ok], rng)
+    assert w <= 5.0, f"{w} units at {at}"
