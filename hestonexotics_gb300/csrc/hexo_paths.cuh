@@ -19,7 +19,7 @@
 #include <stdint.h>
 #include "hexo_types.h"
 #include "hexo_device.cuh"
-#include "hexo_ds.cuh"
+#include "hexo_f32.cuh"
 #include "hexo_f64.cuh"
 
 namespace hexo {
@@ -83,57 +83,6 @@ __device__ __forceinline__ bool qe_step(PathVars<false> &pv, const SegDesc &sg, 
     return quad;
 }
 
-// The FP32 form's branches, m and hs = s^2/2 in double-single, m^2 = p + e.
-// As in the FP64 form (hexo_f64.cuh) the quadratic branch is (sqrt(c) + z
-// sqrt(a))^2 with c = sqrt(m^2 - hs) and a = hs / (m + c): 55 instructions and
-// four MUFU, against 95 for a (b + z)^2 in the reference's order, and no less
-// exact (relative error 2^-45 rms, 2^-44.5 before, the same largest).  The
-// roots and the quotient between stay unnormalised: their low parts are below
-// 2^-22 of the high ones, and what that adds to the next correction is below
-// the rounding that remains.
-__device__ __forceinline__ ds::F2 variance_quadratic(ds::F2 m, ds::F2 hs, float p, float e, float z) {
-    const float D = __fsub_rn(p, hs.h);                                  // m^2 - hs > m^2 / 4
-    const float Dl = __fadd_rn(__fsub_rn(__fsub_rn(p, D), hs.h), __fsub_rn(e, hs.l));
-    const float r1 = ds::rsqrt_approx(D), c = __fmul_rn(D, r1);
-    const float cl = __fmul_rn(__fadd_rn(__fmaf_rn(-c, c, D), Dl), __fmul_rn(0.5f, r1));
-    const float r2 = ds::rsqrt_approx(c), b = __fmul_rn(c, r2);          // sqrt(c)
-    const float bl = __fmul_rn(__fadd_rn(__fmaf_rn(-b, b, c), cl), __fmul_rn(0.5f, r2));
-    const float g = __fadd_rn(m.h, c);                                   // m + c, m >= c
-    const float gl = __fadd_rn(__fsub_rn(c, __fsub_rn(g, m.h)), __fadd_rn(m.l, cl));
-    const float rg = ds::rcp_approx(g), a = __fmul_rn(hs.h, rg);
-    const float al = __fmul_rn(__fmaf_rn(-a, gl, __fadd_rn(__fmaf_rn(-a, g, hs.h), hs.l)), rg);
-    const float r3 = ds::rsqrt_approx(a), s = __fmul_rn(a, r3);          // sqrt(a)
-    const float sl = __fmul_rn(__fadd_rn(__fmaf_rn(-s, s, a), al), __fmul_rn(0.5f, r3));
-    const float q = __fmul_rn(z, s), ql = __fmaf_rn(z, sl, __fmaf_rn(z, s, -q));
-    const ds::F2 w = ds::two_sum(b, q);
-    return ds::sqr(ds::fast_two_sum(w.h, __fadd_rn(w.l, __fadd_rn(bl, ql))));
-}
-
-// -m Y log(Y (1 - U)), Y = (hs + m^2/2) / m^2, 1 - U = (2^64 - w) 2^-64 from
-// the whole word, or 0 where p >= U: that is where Y (1 - U) >= 1, since Y =
-// 1 / (1 - p).  The value is continuous there, so it does not matter that the
-// FP64 form may round a tie the other way.  In double-single like the
-// quadratic branch: a float-size error here would move later branch
-// decisions.
-__device__ __forceinline__ ds::F2 variance_exponential(ds::F2 m, ds::F2 hs, float p, float e, uint64_t uw,
-                                                       const ds::LogTab *ltab) {
-    const float W = __fmaf_rn(0.5f, p, hs.h);                            // hs >= 0.75 m^2
-    const float Wl = __fadd_rn(__fmaf_rn(0.5f, p, __fsub_rn(hs.h, W)), __fmaf_rn(0.5f, e, hs.l));
-    const float rp = ds::rcp_approx(p), y = __fmul_rn(W, rp);
-    const float yl = __fmul_rn(__fmaf_rn(-y, e, __fadd_rn(__fmaf_rn(-y, p, W), Wl)), rp);
-    const ds::F2 om = ds::from_u64_2m64(0ull - uw);
-    const float x = __fmul_rn(y, om.h);
-    const ds::F2 X = ds::fast_two_sum(x, __fmaf_rn(yl, om.h, __fmaf_rn(y, om.l, __fmaf_rn(y, om.h, -x))));
-    ds::F2 vn{0.0f, 0.0f};
-    if (uw != 0ull && (X.h < 1.0f || (X.h == 1.0f && X.l < 0.0f))) {     // U = 0 is never above p
-        const float mY = __fmul_rn(m.h, y);
-        const ds::F2 M{mY, __fmaf_rn(m.l, y, __fmaf_rn(m.h, yl, __fmaf_rn(m.h, y, -mY)))};
-        const ds::F2 v1 = ds::mul(M, ds::neg(ds::log(X, ltab)));
-        if (v1.h > 0.0f) vn = v1;
-    }
-    return vn;
-}
-
 // One QE step, FP32 form: the same scheme and draws; the variance in
 // double-single (m = v disc + m0 and s^2/2 = v cA/2 + cB/2, algebraically the
 // reference's tpp:59-60), everything else in float; returns whether it took
@@ -158,8 +107,8 @@ __device__ __forceinline__ bool qe_step(PathVars<true> &pv, const SegDesc &sg, d
     uint64_t uw = 0;
     dev::draw_commit(g, c, r, dp, quad, z1, uw, z2);
     ds::F2 vn;
-    if (quad) vn = variance_quadratic(m, hs, p, e, z1);
-    else vn = variance_exponential(m, hs, p, e, uw, ltab);
+    if (quad) vn = f32::variance_quadratic(m, hs, p, e, z1);
+    else vn = f32::variance_exponential(m, hs, p, e, uw, ltab);
     pv.vd = vn;
     pv.v = vn.h;
     // K1 v + K2 vn = c (v + vn) + (rho/sigma)(vn - v): the second part
