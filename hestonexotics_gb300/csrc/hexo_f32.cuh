@@ -6,21 +6,26 @@
 namespace hexo {
 namespace f32 {
 
-// The FP32 form's branches, m and hs = s^2/2 in double-single, m^2 = p + e.
+// The two branches take m and hs = s^2/2 in double-single and m^2 = p + e.
 // As in the FP64 form (hexo_f64.cuh) the quadratic branch is (sqrt(c) + z
-// sqrt(a))^2 with c = sqrt(m^2 - hs) and a = hs / (m + c): 55 instructions and
-// four MUFU, against 95 for a (b + z)^2 in the reference's order, and no less
-// exact (relative error 2^-45 rms, 2^-44.5 before, the same largest).  The
-// roots and the quotient between stay unnormalised: their low parts are below
-// 2^-22 of the high ones, and what that adds to the next correction is below
-// the rounding that remains.
+// sqrt(a))^2 with c = sqrt(m^2 - hs) and a = hs / (m + c): 60 instructions and
+// four MUFU, against 95 for a (b + z)^2 in the reference's order.  The roots and
+// the quotient between stay unnormalised.  A correction's own error is the
+// square of what it corrects, 2^-24.5 of a MUFU's product: c and sqrt(c), which
+// every result is made of, are corrected once as floats first, five
+// instructions that take the branch's error from 2^-46.55 to 2^-47.57 rms of
+// its terms for small Psi and from 2^-46.90 to 2^-47.65 around Psi = 1.2 (the
+// reference's order in double-single: 2^-46.68 and 2^-47.25; all measured on the
+// device against 113 bits).
 __device__ __forceinline__ ds::F2 variance_quadratic(ds::F2 m, ds::F2 hs, float p, float e, float z) {
     const float D = __fsub_rn(p, hs.h);                                  // m^2 - hs > m^2 / 4
     const float Dl = __fadd_rn(__fsub_rn(__fsub_rn(p, D), hs.h), __fsub_rn(e, hs.l));
-    const float r1 = ds::rsqrt_approx(D), c = __fmul_rn(D, r1);
-    const float cl = __fmul_rn(__fadd_rn(__fmaf_rn(-c, c, D), Dl), __fmul_rn(0.5f, r1));
-    const float r2 = ds::rsqrt_approx(c), b = __fmul_rn(c, r2);          // sqrt(c)
-    const float bl = __fmul_rn(__fadd_rn(__fmaf_rn(-b, b, c), cl), __fmul_rn(0.5f, r2));
+    const float r1 = ds::rsqrt_approx(D), h1 = __fmul_rn(0.5f, r1), c0 = __fmul_rn(D, r1);
+    const float c = __fmaf_rn(__fadd_rn(__fmaf_rn(-c0, c0, D), Dl), h1, c0);
+    const float cl = __fmul_rn(__fadd_rn(__fmaf_rn(-c, c, D), Dl), h1);
+    const float r2 = ds::rsqrt_approx(c), h2 = __fmul_rn(0.5f, r2), b0 = __fmul_rn(c, r2);
+    const float b = __fmaf_rn(__fmaf_rn(-b0, b0, c), h2, b0);            // sqrt(c)
+    const float bl = __fmul_rn(__fadd_rn(__fmaf_rn(-b, b, c), cl), h2);
     const float g = __fadd_rn(m.h, c);                                   // m + c, m >= c
     const float gl = __fadd_rn(__fsub_rn(c, __fsub_rn(g, m.h)), __fadd_rn(m.l, cl));
     const float rg = ds::rcp_approx(g), a = __fmul_rn(hs.h, rg);

@@ -1,10 +1,11 @@
-"""The FP64 form's own roots, reciprocals and exponential, on the host (CPU).
+"""The path kernels' own arithmetic on the host (CPU): the FP64 form's roots,
+reciprocals, exponential and variance, the FP32 form's variance.
 
-csrc/hexo_f64.cuh uses only integer and individually rounded operations, so it
-compiles for the host (tests/device_math/host_device.h) and gives the device's
-results there but for the two approximate instructions, whose results are the
-correctly rounded ones moved by -1, 0 or 1 unit of the last place: a function
-has to keep its bound with each of those seeds.
+csrc/hexo_f64.cuh and hexo_f32.cuh use only integer and individually rounded
+operations, so they compile for the host (tests/device_math/host_device.h) and
+give the device's results there but for the two approximate instructions, whose
+results are the correctly rounded ones moved by -1, 0 or 1 unit of the last
+place: a function has to keep its bound with each of those seeds.
 """
 import ctypes as C
 import shutil
@@ -18,17 +19,20 @@ from conftest import ROOT
 FN = {"recip": 0, "root": 1, "exp": 2}
 
 
-@pytest.fixture(scope="module")
-def lib(tmp_path_factory):
+def build(name, out):
     if shutil.which("g++") is None:
         pytest.skip("no host compiler")
-    so = tmp_path_factory.mktemp("device_math") / "f64_host.so"
     r = subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-fconstexpr-ops-limit=200000000", "-shared",
                         "-fPIC", "-I", str(ROOT / "hestonexotics_gb300" / "csrc"),
-                        str(ROOT / "tests" / "device_math" / "f64_host.cpp"), "-o", str(so)],
+                        str(ROOT / "tests" / "device_math" / f"{name}.cpp"), "-o", str(out / f"{name}.so")],
                        capture_output=True, text=True)
     assert r.returncode == 0, r.stderr[-4000:]
-    lib = C.CDLL(str(so))
+    return C.CDLL(str(out / f"{name}.so"))
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    lib = build("f64_host", tmp_path_factory.mktemp("device_math"))
     lib.f64_worst_ulp.restype = lib.f64_worst_variance.restype = C.c_double
     return lib
 
@@ -113,3 +117,29 @@ def test_next_variance_over_its_ranges(variance, lo, hi, seed):
     ok = np.abs(lr + 2 * lm) < 60
     w, near, at = variance(seed, 2.0 ** lm[ok], 2.0 ** (lr + 2 * lm)[ok], rng)
     assert w <= 5.0, f"{w} units at {at}"
+
+
+@pytest.fixture(scope="module")
+def f32_rms(tmp_path_factory):
+    lib = build("f32_host", tmp_path_factory.mktemp("device_math_f32"))
+    lib.f32_rms_variance.restype = C.c_double
+
+    def rms(seed, lo, hi):   # log2 of the error, for Psi = s^2/m^2 from 2^lo to 2^hi
+        rng, n = np.random.default_rng(6), 150000
+        m = 2.0 ** rng.uniform(-14, 1, n)
+        s2 = 2.0 ** rng.uniform(lo, hi, n) * m * m
+        z, x = rng.standard_normal(n).astype(np.float32), rng.random(n) / np.maximum(0.5 + 0.5 * s2 / (m * m), 1.0)
+        uw = np.uint64(0) - np.maximum(x * 2.0 ** 64, 1.0).astype(np.uint64)
+        p = lambda a: np.ascontiguousarray(a).ctypes.data_as(C.c_void_p)
+        return np.log2(lib.f32_rms_variance(seed, C.c_uint64(n), p(m), p(s2), p(z), p(uw)))
+    return rms
+
+
+# The reference's order of operations a (b + z)^2, evaluated in normalised double-single steps, has these errors on
+# the same steps (correctly rounded seeds; seeds a unit off); the branch must not be less exact.
+@pytest.mark.parametrize("lo,hi,exact_seed,seed_off", [(-30, -10, -47.13, -44.54), (-10, -3, -47.24, -44.62),
+                                                       (-3, 0.58, -47.51, -45.03)])
+def test_fp32_quadratic_branch(f32_rms, lo, hi, exact_seed, seed_off):
+    assert f32_rms(0, lo, hi) <= exact_seed
+    assert f32_rms(1, lo, hi) <= seed_off
+    assert f32_rms(-1, lo, hi) <= seed_off
