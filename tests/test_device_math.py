@@ -143,3 +143,11 @@ def test_fp32_quadratic_branch(f32_rms, lo, hi, exact_seed, seed_off):
     assert f32_rms(0, lo, hi) <= exact_seed
     assert f32_rms(1, lo, hi) <= seed_off
     assert f32_rms(-1, lo, hi) <= seed_off
+
+
+# The exponential branch with a logarithm good to 2^-46 of 1: a unit of that from each of r's two parts, the table's
+# and the sums' (2^-44.0 without r's low part in the cubic term).
+@pytest.mark.parametrize("seed", [-1, 0, 1])
+@pytest.mark.parametrize("lo,hi", [(0.6, 2), (2, 8), (8, 20)])
+def test_fp32_exponential_branch(f32_rms, lo, hi, seed):
+    assert f32_rms(seed, lo, hi) <= -45.5
