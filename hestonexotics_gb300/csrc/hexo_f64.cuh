@@ -368,18 +368,24 @@ __device__ __forceinline__ bool in_range(double m, double s2) {
 }
 
 // Whether the step takes the quadratic branch, s2 < 1.5 m^2 (Psi < PSI_C,
-// HSimulation.tpp:61-63): in float while in range and unless the two are
-// within 2^-20.  The exact comparison is a call so that it is not computed
-// ahead of the branch (three FP64 instructions in every step).
+// HSimulation.tpp:61-63), while in range: in float unless the two are within
+// 2^-20.  The exact comparison is a call so that it is not computed ahead of
+// the branch (three FP64 instructions in every step).
 static __device__ __noinline__ bool quadratic_exact(double m, double s2) {
     return s2 < __dmul_rn(1.5, __dmul_rn(m, m));
 }
-__device__ __forceinline__ bool quadratic(double m, double s2, bool near) {
+__device__ __forceinline__ bool quadratic(double m, double s2) {
     const float mf = head(m), sf = head(s2);
     const float t = __fmul_rn(__fmul_rn(1.5f, mf), mf);
     bool quad = sf < t;
-    if (!near || !(fabsf(__fsub_rn(sf, t)) > __fmul_rn(0x1p-20f, sf))) quad = quadratic_exact(m, s2);
+    if (!(fabsf(__fsub_rn(sf, t)) > __fmul_rn(0x1p-20f, sf))) quad = quadratic_exact(m, s2);
     return quad;
+}
+// The same outside in_range, on the mean in the reference's order of
+// operations, as variance_wide takes it (where exp(-kappa dt) rounds to 1 the
+// two means can differ by all of v).
+static __device__ __noinline__ bool quadratic_wide(double v, double theta, double disc, double s2) {
+    return quadratic_exact(__fma_rn(__dsub_rn(v, theta), disc, theta), s2);
 }
 
 // The quadratic branch a (b + z)^2 (HSimulation.tpp:64-68).  Its a and b

@@ -65,7 +65,7 @@ __device__ __forceinline__ bool qe_step(PathVars<false> &pv, const SegDesc &sg, 
     const double m = __fma_rn(v, sg.disc, sg.m0);                            // tpp:59
     const double s2 = fabs(__fma_rn(v, sg.cA, sg.cB));                       // tpp:60
     const bool near = f64::in_range(m, s2);
-    const bool quad = f64::quadratic(m, s2, near);
+    const bool quad = near ? f64::quadratic(m, s2) : f64::quadratic_wide(v, theta, sg.disc, s2);
     if (dev::draw_prepare<false>(g, c, r, ws, quad)) dp = dev::draw_prefetch(c, r);
     float z1 = 0.0f, z2;                                                     // draw order, tpp:67,72,80
     uint64_t uw = 0;

@@ -52,7 +52,7 @@ extern "C" double f64_worst_variance(int seed_ulp, uint64_t n, const double *m, 
     double worst = 0.0;
     for (uint64_t i = 0; i < n; ++i) {
         near[i] = f64::in_range(m[i], s2[i]);
-        const bool quad = f64::quadratic(m[i], s2[i], near[i]);
+        const bool quad = near[i] ? f64::quadratic(m[i], s2[i]) : f64::quadratic_wide(m[i], 0.0, 1.0, s2[i]);
         const double got = !near[i] ? f64::variance_wide(m[i], 0.0, 1.0, s2[i], quad, z[i], uw[i])
                            : quad   ? f64::variance_quadratic(m[i], s2[i], z[i])
                                     : f64::variance_exponential(m[i], s2[i], uw[i]);

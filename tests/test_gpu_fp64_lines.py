@@ -55,3 +55,19 @@ def test_prices_on_either_side(engine, oracle, name):
     assert np.isfinite(want).all()
     magnified = steps * abs(rho) / sigma * max(v0, theta) * 8 * 2.0 ** -53
     np.testing.assert_allclose(price, want, rtol=1e-10, atol=S0 * (1e-12 + magnified))
+
+
+@pytest.mark.parametrize("steps,T", [(1, 0.5), (30, 0.001)])
+@pytest.mark.parametrize("v0,theta,kappa", [(1e-20, 0.04, 1e-17), (1e-30, 50.0, 1e-18), (1e-12, 1e6, 1e-17)])
+def test_reversion_below_a_last_bit(engine, oracle, v0, theta, kappa, steps, T):
+    # exp(-kappa dt) is 1: the reference's theta + (v - theta) disc loses v0 beside theta, the mean and s^2 are 0, and
+    # the variance stays 0.  Outside its own functions' range the step has to branch on that mean, not on v0's.
+    p = (v0, theta, -0.5, kappa, 0.3, 0.01, 0.0)
+    assert np.exp(-kappa * T / steps) == 1.0 and (v0 - theta) + theta == 0.0
+    K = np.array([0.0, 60.0, 95.0, 100.0] * 2)
+    kind = np.repeat([E.ASIAN, E.EUROPEAN], 4).astype(np.uint32)
+    opts = E.Options(K, T, kind)
+    price, _ = engine.price(E.Params(*p), 100.0, opts, E.Config(n_paths=200, steps=steps, seed=3))
+    want, _, _ = oracle.price_paths(np.array(p), 100.0, K, opts.T, kind.astype(np.uint8), n_default=200, steps=steps, seed=3)
+    assert want[4] > 99.0   # a European call struck at 0 is the spot
+    np.testing.assert_allclose(price, want, rtol=1e-10, atol=1e-10)
