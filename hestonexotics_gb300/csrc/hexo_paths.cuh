@@ -29,7 +29,8 @@ namespace hexo {
 // its operand is normal, and the other form spends three instructions on
 // operands that are not).
 __device__ __forceinline__ float fsqrt_fast(float x) { return __fmul_rn(x, ds::rsqrt_approx(fmaxf(x, 1e-30f))); }
-// exp(x) as __expf, results below 2^-126 as 0.
+// exp(x) as 2^(x log2 e) by the MUFU; results below 2^-126 are 0 (a spot so far down is 2^-78 of
+// the payoffs' last unit).
 __device__ __forceinline__ float exp_fast(float x) {
     float r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__fmul_rn(x, 1.4426950408889634f)));

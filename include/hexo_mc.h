@@ -316,7 +316,8 @@ hexo_status hexo_swift_params_dynamic(const hexo_params *p, double tau, double S
  * SWIFT.cpp:51-52): direct sums cost O(J (k2 - k1)), the FFT O(J log J);
  * both give the same prices to rounding. */
 typedef enum hexo_swift_method {
-    HEXO_SWIFT_AUTO = 0,    /* the FFT from J = 16 frequencies on, direct sums below */
+    HEXO_SWIFT_AUTO = 0,    /* the FFT from J = 16 frequencies on (1024 where upper > 12, see
+                               hexo_swift_params), direct sums below */
     HEXO_SWIFT_DIRECT = 1,  /* direct sums */
     HEXO_SWIFT_FFT = 2      /* FFT of length 2J */
 } hexo_swift_method;
