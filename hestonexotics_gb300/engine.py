@@ -402,8 +402,11 @@ class Engine:
         """requests: [(Params, S, [(tau, strikes), ...]), ...], priced in one call."""
         # one array each for all strikes, prices and gradients, and one of chain records (a record,
         # three arrays and four casts per chain took ten microseconds each, more than its pricing)
-        flat = [(float(tau), np.ascontiguousarray(K, dtype=np.float64)) for _, _, chains in requests for tau, K in chains]
-        Ks = [K for _, K in flat]
+        taus, Ks = [], []
+        for _, _, chains in requests:
+            for tau, K in chains:
+                taus.append(float(tau))
+                Ks.append(np.ascontiguousarray(K, dtype=np.float64))
         ns = np.array([len(K) for K in Ks], dtype=np.int64)
         ends = np.cumsum(ns)
         total = int(ends[-1]) if len(ns) else 0
@@ -413,7 +416,7 @@ class Engine:
         at = (ends - ns).astype(np.uint64)
         arr = np.zeros(max(1, len(Ks)), dtype=_CHAIN_DTYPE)
         rec = arr[:len(Ks)]
-        rec["tau"] = [tau for tau, _ in flat]
+        rec["tau"] = taus
         rec["strikes"] = np.uint64(strikes.ctypes.data) + 8 * at
         rec["n"] = ns
         # converted as ctypes fields: numpy would refuse a method below 0 and take None, text or arrays for a number
