@@ -45,12 +45,6 @@ __device__ __forceinline__ F2 mul_f(F2 x, float f) {
     e = __fmaf_rn(x.l, f, e);
     return fast_two_sum(p, e);
 }
-__device__ __forceinline__ F2 sqr(F2 x) {
-    const float p = __fmul_rn(x.h, x.h);
-    float e = __fmaf_rn(x.h, x.h, -p);
-    e = __fmaf_rn(__fadd_rn(x.h, x.h), x.l, e);
-    return fast_two_sum(p, e);
-}
 // Approximate MUFU reciprocal and reciprocal square root.  Each is a fixed
 // function of its input, so results stay reproducible; a Newton-style
 // correction with the exact remainder brings what is made of them to

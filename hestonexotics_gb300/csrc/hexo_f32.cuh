@@ -8,15 +8,15 @@ namespace f32 {
 
 // The two branches take m and hs = s^2/2 in double-single and m^2 = p + e.
 // As in the FP64 form (hexo_f64.cuh) the quadratic branch is (sqrt(c) + z
-// sqrt(a))^2 with c = sqrt(m^2 - hs) and a = hs / (m + c): 60 instructions and
-// four MUFU, against 95 for a (b + z)^2 in the reference's order.  The roots and
-// the quotient between stay unnormalised.  A correction's own error is the
-// square of what it corrects, 2^-24.5 of a MUFU's product: c and sqrt(c), which
-// every result is made of, are corrected once as floats first, five
-// instructions that take the branch's error from 2^-46.55 to 2^-47.57 rms of
-// its terms for small Psi and from 2^-46.90 to 2^-47.65 around Psi = 1.2 (the
-// reference's order in double-single: 2^-46.68 and 2^-47.25; all measured on the
-// device against 113 bits).
+// sqrt(a))^2 with c = sqrt(m^2 - hs) and a = hs / (m + c): 57 instructions and
+// four MUFU, against 95 for a (b + z)^2 in the reference's order.  What comes
+// between stays unnormalised, the square taking its low part's square along.  A
+// correction's own error is the square of what it corrects, 2^-24.5 of a
+// MUFU's product: c and sqrt(c), which every result is made of, are corrected
+// once as floats first.  Error, rms of the result's terms, measured on the device
+// against 113 bits: 2^-47.34 for small Psi, 2^-47.60 up to 1, 2^-47.49 beyond
+// (without the corrections 2^-46.55, 2^-46.92 and 2^-46.90; the reference's order
+// in normalised double-single steps 2^-46.68, 2^-47.11 and 2^-47.25).
 __device__ __forceinline__ ds::F2 variance_quadratic(ds::F2 m, ds::F2 hs, float p, float e, float z) {
     const float D = __fsub_rn(p, hs.h);                                  // m^2 - hs > m^2 / 4
     const float Dl = __fadd_rn(__fsub_rn(__fsub_rn(p, D), hs.h), __fsub_rn(e, hs.l));
@@ -34,7 +34,8 @@ __device__ __forceinline__ ds::F2 variance_quadratic(ds::F2 m, ds::F2 hs, float 
     const float sl = __fmul_rn(__fadd_rn(__fmaf_rn(-s, s, a), al), __fmul_rn(0.5f, r3));
     const float q = __fmul_rn(z, s), ql = __fmaf_rn(z, sl, __fmaf_rn(z, s, -q));
     const ds::F2 w = ds::two_sum(b, q);
-    return ds::sqr(ds::fast_two_sum(w.h, __fadd_rn(w.l, __fadd_rn(bl, ql))));
+    const float wl = __fadd_rn(w.l, __fadd_rn(bl, ql)), v = __fmul_rn(w.h, w.h);
+    return ds::fast_two_sum(v, __fmaf_rn(__fmaf_rn(2.0f, w.h, wl), wl, __fmaf_rn(w.h, w.h, -v)));
 }
 
 // -m Y log(Y (1 - U)), Y = (hs + m^2/2) / m^2, 1 - U = (2^64 - w) 2^-64 from
