@@ -56,8 +56,8 @@ struct PathVars {
 // took the quadratic branch.  As the reference writes it, a step is about 100
 // FP64 instructions, and that pipe bounds it; with the roots, quotients, log
 // and exp of hexo_f64.cuh it is 14 (quadratic) or 10 (exponential) with the
-// trapezoid: 64-set batch at 1/128 of its paths 546 -> 90.6 ms, plain Asian
-// 4.46 -> 0.74 ms.
+// trapezoid: 64-set batch at 1/128 of its paths 546 -> 90.1 ms, plain Asian
+// 4.46 -> 0.73 ms.
 __device__ __forceinline__ bool qe_step(PathVars<false> &pv, const SegDesc &sg, const double &theta, dev::Shishua &g,
                                         dev::RngLane &c, const dev::Ring &r, const dev::WarpScratch &ws,
                                         const f64::ExpTab *etab) {
